@@ -92,7 +92,7 @@ constexpr int kBookWarpFloats = 1024 + kBookLsFloats + kBookAssetFloats + 2 * kB
 // transpose tile after the per-warp area.  Pairing gained nothing at d = 9 and cost 4-7 % in the
 // d 5-8 class (d = 7, and d = 8 through the larger kernel), so those keep single tiles.
 __host__ __device__ constexpr bool book_pair_tiles(int d) { return d == 11 || d == 12; }
-// After them, the Sobol start words a warp carries from group to group of a chunk (sobol_tile): one
+// After them, the Sobol start words a warp carries from group to group of a chunk (sobol_tile_plain): one
 // 32-word slot per tile for a path's first kBookCarryTiles tiles (a chunk's later tiles walk their
 // start word), sized so that the basket classes keep three resident CTAs per SM; the single-asset
 // class carries paths of up to kBookSingleCarryTiles tiles whole.
@@ -280,7 +280,7 @@ __device__ __forceinline__ void book_chunk(const BookArgs& a, const BookSpec& s,
     const float K = o.K, disc = o.disc;
     const bool has_c = nc > 0;
     const int dstride = a.dstride[s.level];
-    const uint32_t* dr = a.dirs[s.level] + (size_t)r * 33 * (size_t)dstride;
+    const uint32_t* dr = a.dirs[s.level] + (size_t)r * kPlainRows * (size_t)dstride;
     const int Dt = nf * D;
     const uint64_t pend = (uint64_t)s.offset + s.n_points;
     const float4* L4 = reinterpret_cast<const float4*>(Ls);
@@ -289,7 +289,7 @@ __device__ __forceinline__ void book_chunk(const BookArgs& a, const BookSpec& s,
         const int Q = 32 / Dt, qj = lane / Dt, dj = lane - qj * Dt;
         for (uint64_t g = gb; g < ge; g += Q) {
             const uint64_t gl = g + (uint64_t)qj;
-            sobol_tile(dr, dstride, dj, qj < Q && gl < ge, gl, a.u_cap, buf, lane);
+            sobol_tile_plain(dr, dstride, dj, qj < Q && gl < ge, gl, a.u_cap, buf, lane);
             __syncwarp();
             for (int q = 0; q < Q && g + q < ge; q++) {
                 P path;
@@ -317,9 +317,9 @@ __device__ __forceinline__ void book_chunk(const BookArgs& a, const BookSpec& s,
             for (int k0 = 0, t = 0; k0 < nf; k0 += S2, t += 2) {
                 const int dim = k0 * D + lane;
                 const bool cont = g != gb;
-                sobol_tile(dr, dstride, dim, dim < Dt, g, a.u_cap, buf, lane,
+                sobol_tile_plain(dr, dstride, dim, dim < Dt, g, a.u_cap, buf, lane,
                            t < kBookCarryTiles ? carry + 32 * t + lane : nullptr, cont);
-                sobol_tile(dr, dstride, dim + 32, lane < W2 - 32 && dim + 32 < Dt, g, a.u_cap, buf2, lane,
+                sobol_tile_plain(dr, dstride, dim + 32, lane < W2 - 32 && dim + 32 < Dt, g, a.u_cap, buf2, lane,
                            t + 1 < kBookCarryTiles ? carry + 32 * (t + 1) + lane : nullptr, cont);
                 __syncwarp();
                 const float4* rowA = reinterpret_cast<const float4*>(buf + lane * 32);
@@ -352,7 +352,7 @@ __device__ __forceinline__ void book_chunk(const BookArgs& a, const BookSpec& s,
             path.init(sg);
             for (int k0 = 0, t = 0; k0 < nf; k0 += S, t++) {
                 const int dim = k0 * D + lane;
-                sobol_tile(dr, dstride, dim, lane < W && dim < Dt, g, a.u_cap, buf, lane,
+                sobol_tile_plain(dr, dstride, dim, lane < W && dim < Dt, g, a.u_cap, buf, lane,
                            t < kBookCarryTiles ? carry + 32 * t + lane : nullptr, g != gb);
                 __syncwarp();
                 // this path's row of the tile, read per step as float4 chunks (conflict-free in
@@ -437,7 +437,7 @@ __device__ __forceinline__ void single_chunk(const KParams& kp, const BookSpec& 
         C cons;
         cons.init(kp);
         cons.bind(r, n);
-        run_group<GEN_SOBOL, NOISE_RAW>(kp, cons, dr, 0u, h, n, buf, nullptr, lane, carry, h != gb);
+        run_group<GEN_SOBOL, NOISE_RAW, C, true>(kp, cons, dr, 0u, h, n, buf, nullptr, lane, carry, h != gb);
         float y[C::NST];
         cons.finish(kp, y);
         if (n >= s.offset && n < pend) acc.add(y);
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_book_single(const __grid_con
         const uint64_t gend = ((uint64_t)s.offset + s.n_points - 1) / 32 + 1;
         const uint64_t gb = (s.offset >> 5) + (uint64_t)j * (uint64_t)s.gpc;
         const uint64_t ge = min(gb + (uint64_t)s.gpc, gend);
-        const uint32_t* dr = a.dirs[s.level] + (size_t)r * 33 * (size_t)a.dstride[s.level];
+        const uint32_t* dr = a.dirs[s.level] + (size_t)r * kPlainRows * (size_t)a.dstride[s.level];
         double* rec = a.records + (size_t)c * kBookNST;
         switch (kp.model) {
             case MOD_HESTON: single_chunk_pay<MOD_HESTON>(kp, s, r, gb, ge, dr, buf, rec, lane); break;
@@ -756,8 +756,8 @@ struct BookRunner {
         for (int l = 0; l <= max_L_all; l++) {
             dstride[l] = (int)(dmax * nfine(l));
             dirs[l] = &E.ws(1 + l).xbuf[4];
-            uint32_t* t = (uint32_t*)grow(*dirs[l], sizeof(uint32_t) * (size_t)R * 33 * dstride[l]);
-            launch_prescramble(E.d_dv, qc.salt_base + (uint32_t)(l * R), R, dstride[l], t, s0);
+            uint32_t* t = (uint32_t*)grow(*dirs[l], sizeof(uint32_t) * (size_t)R * kPlainRows * dstride[l]);
+            launch_prescramble_plain(E.d_dv, qc.salt_base + (uint32_t)(l * R), R, dstride[l], t, s0);
         }
         for (size_t q = 0; q < kps.size(); q++) {
             const int l = (int)(q % kBookMaxLevels);

@@ -633,7 +633,7 @@ static void sobol_export(uint32_t salt, int dim0, int nd, uint32_t offset, int64
     Workspace& ws = engine().ws(0);
     const int D = dim0 + nd;
     uint32_t* tab = (uint32_t*)ws.dirs.ensure(sizeof(uint32_t) * 33 * (size_t)D);
-    launch_prescramble(engine().d_dv, salt, 1, D, tab, ws.stream);
+    launch_prescramble_plain(engine().d_dv, salt, 1, D, tab, ws.stream);
     ws.dirs_R = -1;   // table no longer matches any cached pass layout
     const size_t bytes = sizeof(uint32_t) * (size_t)nd * (size_t)n;
     void* d = ws.dump.ensure(bytes);

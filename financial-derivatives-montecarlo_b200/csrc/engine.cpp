@@ -389,6 +389,24 @@ const TuneState* tune_state(uint64_t key) {
     return it == engine().tune.end() ? nullptr : &it->second;
 }
 
+// The workspace's scrambled direction words for R salts from salt0 and D dimensions, formed again when
+// the last table on it was another one.
+const uint32_t* direction_table(Workspace& ws, uint32_t salt0, int R, int D, bool plain) {
+    Engine& E = engine();
+    if (!(ws.dirs_salt0 == salt0 && ws.dirs_R == R && ws.dirs_D == D && ws.dirs_plain == plain)) {
+        ws.dirs_R = -1;
+        const size_t rows = plain ? kPlainRows : kDirRows;
+        uint32_t* d = (uint32_t*)ws.dirs.ensure(sizeof(uint32_t) * (size_t)R * rows * D);
+        (plain ? launch_prescramble_plain : launch_prescramble)(E.d_dv, salt0, R, D, d, ws.stream);
+        E.launches++;
+        ws.dirs_salt0 = salt0;
+        ws.dirs_R = R;
+        ws.dirs_D = D;
+        ws.dirs_plain = plain;
+    }
+    return (const uint32_t*)ws.dirs.p;
+}
+
 void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     Engine& E = engine();
     MCQ_REQUIRE(a.m && a.p, MCQ_ERR_INVALID, "null model or payoff");
@@ -444,7 +462,7 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
         return;
     }
 
-    const void* fn = a.dump ? lookup_misc(a.gen, a.noise, a.est, k.model, nb, true)
+    const void* fn = a.dump ? lookup_dump(a.gen, a.noise, !(a.flags & MCQ_FLAG_DUMP_PRICED))
                             : lookup_pass(a.gen, knoise, a.est, k.model, a.p->kind, nb);
     // short raw-ordered Sobol paths: 32 / D path groups per tile instead of one
     const void* packed = nullptr;
@@ -499,15 +517,7 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     k.G = G;
 
     if (a.gen == GEN_SOBOL) {
-        if (!(ws.dirs_salt0 == a.salt0 && ws.dirs_R == a.R && ws.dirs_D == D)) {
-            uint32_t* d = (uint32_t*)ws.dirs.ensure(sizeof(uint32_t) * (size_t)a.R * 33 * D);
-            launch_prescramble(E.d_dv, a.salt0, a.R, D, d, ws.stream);
-            E.launches++;
-            ws.dirs_salt0 = a.salt0;
-            ws.dirs_R = a.R;
-            ws.dirs_D = D;
-        }
-        k.dirs = (const uint32_t*)ws.dirs.p;
+        k.dirs = direction_table(ws, a.salt0, a.R, D, false);
     }
     const int nst = a.dump ? 1 : k.nstat;
     k.nstat = nst;
@@ -519,8 +529,8 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     const int skel = (a.noise == NOISE_BB && D > 32) ? ((D >> 5) + 1) * 32 : 0;
     const int accf = (!a.dump && a.est == EST_COUPLED && (k.model == MOD_BASKET || k.model == MOD_MULTI))
                          ? ((2 * nst + 3) & ~3) : 0;
-    size_t smem = assist ? (size_t)kAssistTeams * kAssistTeamBytes
-                         : (size_t)kWarpsPerBlock * (1024 + skel + accf) * sizeof(float);
+    size_t smem = kTilePad + (assist ? (size_t)kAssistTeams * kAssistTeamBytes
+                                     : (size_t)kWarpsPerBlock * (1024 + skel + accf) * sizeof(float));
     // Sobol start words carried from group to group of an item (one slot per tile a group
     // generates): kept when an item has several groups and the slots leave the kernel's resident
     // blocks per SM unchanged
@@ -559,7 +569,8 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
 void pca_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* d_out) {
     Engine& E = engine();
     const int N = k.D;
-    const void* fn = lookup_pca(k.model, a.p->kind, a.est == EST_COUPLED, a.dump);
+    const void* fn = a.dump ? lookup_pca_dump(!(a.flags & MCQ_FLAG_DUMP_PRICED))
+                            : lookup_pca(k.model, a.p->kind, a.est == EST_COUPLED);
     MCQ_REQUIRE(fn != nullptr, MCQ_ERR_UNSUPPORTED, "no tensor-core PCA kernel for this model / payoff");
     const uint64_t g0 = a.offset >> 5;
     const uint64_t G = ((a.offset + a.n_points - 1) >> 5) - g0 + 1;
@@ -580,15 +591,7 @@ void pca_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* d_out)
     k.n_points = a.n_points;
     k.g0 = g0;
     k.G = G;
-    if (!(ws.dirs_salt0 == a.salt0 && ws.dirs_R == a.R && ws.dirs_D == N)) {
-        uint32_t* d = (uint32_t*)ws.dirs.ensure(sizeof(uint32_t) * (size_t)a.R * 33 * N);
-        launch_prescramble(E.d_dv, a.salt0, a.R, N, d, ws.stream);
-        E.launches++;
-        ws.dirs_salt0 = a.salt0;
-        ws.dirs_R = a.R;
-        ws.dirs_D = N;
-    }
-    k.dirs = (const uint32_t*)ws.dirs.p;
+    k.dirs = direction_table(ws, a.salt0, a.R, N, false);
     const int nst = a.dump ? 1 : k.nstat;
     k.nstat = nst;
     k.partials = (double*)ws.partials.ensure(sizeof(double) * (size_t)k.n_items * pca_warps() * nst);
@@ -690,13 +693,7 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
     const uint64_t ipr = (G + gpi - 1) / gpi;
     k.R = R; k.gpi = (int)gpi; k.items_per_rep = (int)ipr; k.n_items = (int)(ipr * R);
     k.offset = offset; k.n_points = n_points; k.g0 = g0; k.G = G;
-    if (!(ws.dirs_salt0 == salt_base && ws.dirs_R == R && ws.dirs_D == k.D)) {
-        uint32_t* d = (uint32_t*)ws.dirs.ensure(sizeof(uint32_t) * (size_t)R * 33 * k.D);
-        launch_prescramble(E.d_dv, salt_base, R, k.D, d, ws.stream);
-        E.launches++;
-        ws.dirs_salt0 = salt_base; ws.dirs_R = R; ws.dirs_D = k.D;
-    }
-    k.dirs = (const uint32_t*)ws.dirs.p;
+    k.dirs = direction_table(ws, salt_base, R, k.D, true);
     k.nstat = 4;
     k.partials = (double*)ws.partials.ensure(sizeof(double) * (size_t)k.n_items * 4);
     double* d_nodes = nullptr;

@@ -70,6 +70,7 @@ struct Workspace {
     } blas;
     uint32_t dirs_salt0 = 0;
     int dirs_R = -1, dirs_D = -1;
+    bool dirs_plain = false;
     void ensure_stream();
     ~Workspace();
 };
@@ -169,6 +170,8 @@ int noise_dim(const mcq_model& m);
 void fill_params(Workspace& ws, const PassArgs& a, KParams& k);
 int nstat_of(int est);
 int nstat_of(int est, int model_kind);   // basket levels carry per-asset deltas
+// The direction table of a pass on ws.stream: the passes' reduced form, or the plain one (kparams.h).
+const uint32_t* direction_table(Workspace& ws, uint32_t salt0, int R, int D, bool plain);
 // Enqueue one pass on ws.stream; d_out receives [R][nstat] doubles (device).
 void pass_async(Workspace& ws, const PassArgs& a, double* d_out);
 // Tensor-core PCA pass (N in {64, 128, 256}); called by pass_async.

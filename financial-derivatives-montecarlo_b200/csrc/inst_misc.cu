@@ -2,13 +2,7 @@
 namespace mcq {
 
 template <int GEN>
-static const void* misc_gen(int noise, int est, int model, int nb, bool dump) {
-    if (dump) {
-        if (noise == NOISE_RAW) return (const void*)&k_pass<GEN, NOISE_RAW, DumpC>;
-        if (noise == NOISE_BB && GEN == GEN_SOBOL) return (const void*)&k_pass<GEN_SOBOL, NOISE_BB, DumpC>;
-        if (noise == NOISE_PCA && GEN == GEN_SOBOL) return (const void*)&k_pass<GEN_SOBOL, NOISE_PCA, DumpC>;
-        return nullptr;
-    }
+static const void* misc_gen(int noise, int est, int model, int nb) {
     if (noise != NOISE_RAW) return nullptr;
     if (est == EST_CV_ASIAN) return (const void*)&k_pass<GEN, NOISE_RAW, CvAsianC>;
     if (est == EST_CV_DUPIRE) return (const void*)&k_pass<GEN, NOISE_RAW, CvDupireC>;
@@ -44,8 +38,21 @@ static const void* misc_gen(int noise, int est, int model, int nb, bool dump) {
     return nullptr;
 }
 
-const void* lookup_misc(int gen, int noise, int est, int model, int nb, bool dump) {
-    return gen == GEN_SOBOL ? misc_gen<GEN_SOBOL>(noise, est, model, nb, dump)
-                            : misc_gen<GEN_PHILOX>(noise, est, model, nb, dump);
+const void* lookup_misc(int gen, int noise, int est, int model, int nb) {
+    return gen == GEN_SOBOL ? misc_gen<GEN_SOBOL>(noise, est, model, nb)
+                            : misc_gen<GEN_PHILOX>(noise, est, model, nb);
+}
+
+template <bool PARITY>
+static const void* dump_noise(int noise) {
+    if (noise == NOISE_RAW) return (const void*)&k_pass<GEN_SOBOL, NOISE_RAW, DumpC<PARITY>>;
+    if (noise == NOISE_BB) return (const void*)&k_pass<GEN_SOBOL, NOISE_BB, DumpC<PARITY>>;
+    if (noise == NOISE_PCA) return (const void*)&k_pass<GEN_SOBOL, NOISE_PCA, DumpC<PARITY>>;
+    return nullptr;
+}
+
+const void* lookup_dump(int gen, int noise, bool parity) {
+    if (gen == GEN_SOBOL) return parity ? dump_noise<true>(noise) : dump_noise<false>(noise);
+    return noise == NOISE_RAW ? (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, DumpC<false>> : nullptr;
 }
 }  // namespace mcq

@@ -1,14 +1,14 @@
 #include "inst_common.cuh"
 namespace mcq {
 // Brownian-bridge passes with uniform window weights (NOISE_BB_UNI): plain at 3 and 4 resident CTAs
-// per SM with the tile generator's block loop rolled, and at 3 with it unrolled (the autotuner's
-// variants; 2 CTAs lost to 3 and 4 on every measured workload), coupled at the default 2.
-template <int MINB, int GU = 1>
+// per SM (the autotuner's variants; 2 CTAs lost to 3 and 4 on every measured workload), coupled at the
+// default 2.
+template <int MINB>
 static const void* bbu_plain(int model, int pay) {
     switch (model) {
-        case MOD_GBM: return pick_payoff<GEN_SOBOL, NOISE_BB_UNI, MOD_GBM, false, MINB, GU>(pay);
-        case MOD_DUPIRE: return pick_payoff<GEN_SOBOL, NOISE_BB_UNI, MOD_DUPIRE, false, MINB, GU>(pay);
-        case MOD_LVGRID: return pick_payoff<GEN_SOBOL, NOISE_BB_UNI, MOD_LVGRID, false, MINB, GU>(pay);
+        case MOD_GBM: return pick_payoff<GEN_SOBOL, NOISE_BB_UNI, MOD_GBM, false, MINB>(pay);
+        case MOD_DUPIRE: return pick_payoff<GEN_SOBOL, NOISE_BB_UNI, MOD_DUPIRE, false, MINB>(pay);
+        case MOD_LVGRID: return pick_payoff<GEN_SOBOL, NOISE_BB_UNI, MOD_LVGRID, false, MINB>(pay);
         default: return nullptr;
     }
 }
@@ -24,7 +24,6 @@ const void* lookup_sobol_bbu(int model, int pay, bool coupled, int variant) {
     switch (variant) {
         case 0: return bbu_plain<3>(model, pay);
         case 1: return bbu_plain<4>(model, pay);
-        case 2: return bbu_plain<3, 4>(model, pay);
         default: return nullptr;
     }
 }

@@ -4,7 +4,7 @@
 // For each path (lane) the forward sweep steps S_k -> S_{k+1} = S_k (1 + mu h + sigma_k dW_k),
 // keeps the payoff state and checkpoints S every CK steps (16, 32 or 8: an autotuned launch
 // variant) in shared memory.  The reverse sweep walks the 32-step Sobol tiles backwards: it
-// regenerates the tile's normals (same warp-transposed generator as the pricing pass), recomputes
+// regenerates the tile's normals (the generator's plain form), recomputes
 // each CK-step segment from its checkpoint, and propagates
 //     Sbar_k = Sbar_{k+1} dS_{k+1}/dS_k + dP/dS_k,
 //     mubar += Sbar_{k+1} S_k h,            sigmabar += Sbar_{k+1} dS_{k+1}/dsigma,
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_adjoint(const __grid_constant__
         const int j = item - r * p.items_per_rep;
         const uint64_t gb = p.g0 + (uint64_t)j * (uint64_t)p.gpi;
         const uint64_t ge = min(gb + (uint64_t)p.gpi, gend_all);
-        const uint32_t* dr = p.dirs + (size_t)r * 33 * (size_t)N;
+        const uint32_t* dr = p.dirs + (size_t)r * kPlainRows * (size_t)N;
         Acc<4> acc;
         acc.zero();
         for (uint64_t hg = gb; hg < ge; hg++) {
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_adjoint(const __grid_constant__
             float S = p.S0, ts = 0.f, tot = 0.f, comp = 0.f, mn = p.S0;
             int kmin = 0;
             for (int d0 = 0; d0 < N; d0 += 32) {
-                sobol_tile(dr, N, d0 + lane, true, hg, p.u_cap, buf, lane, carry + d0 + lane, hg != gb ? 1 : 0);
+                sobol_tile_plain(dr, N, d0 + lane, true, hg, p.u_cap, buf, lane, carry + d0 + lane, hg != gb ? 1 : 0);
                 __syncwarp();
                 // the step loops read this lane's row of the tile from shared memory, four steps
                 // per float4 (the swizzled layout makes row reads conflict-free), and stay rolled
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_adjoint(const __grid_constant__
             int vcell = -1;
             float v00 = 0.f, v01 = 0.f, v10 = 0.f, v11 = 0.f;
             for (int d0 = N - 32; d0 >= 0; d0 -= 32) {
-                sobol_tile(dr, N, d0 + lane, true, hg, p.u_cap, buf, lane, carry + d0 + lane, 2);
+                sobol_tile_plain(dr, N, d0 + lane, true, hg, p.u_cap, buf, lane, carry + d0 + lane, 2);
                 __syncwarp();
                 const float4* row4 = reinterpret_cast<const float4*>(buf + lane * 32);
 #pragma unroll 1
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_adjoint_heston(const __grid_con
         const int j = item - r * p.items_per_rep;
         const uint64_t gb = p.g0 + (uint64_t)j * (uint64_t)p.gpi;
         const uint64_t ge = min(gb + (uint64_t)p.gpi, gend_all);
-        const uint32_t* dr = p.dirs + (size_t)r * 33 * (size_t)D;
+        const uint32_t* dr = p.dirs + (size_t)r * kPlainRows * (size_t)D;
         Acc<4> acc;
         acc.zero();
         for (uint64_t hg = gb; hg < ge; hg++) {
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_adjoint_heston(const __grid_con
             for (int t = 0; t < n_tiles; t++) {
                 ckS[t * 32 + lane] = S;
                 ckV[t * 32 + lane] = V;
-                sobol_tile(dr, D, t * 32 + lane, true, hg, p.u_cap, buf, lane);
+                sobol_tile_plain(dr, D, t * 32 + lane, true, hg, p.u_cap, buf, lane);
                 __syncwarp();
                 float z[32];
                 read_row(buf, lane, z);
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_adjoint_heston(const __grid_con
             // ---------------- reverse sweep
             float mubar = 0.f, Vbar = 0.f;
             for (int t = n_tiles - 1; t >= 0; t--) {
-                sobol_tile(dr, D, t * 32 + lane, true, hg, p.u_cap, buf, lane);
+                sobol_tile_plain(dr, D, t * 32 + lane, true, hg, p.u_cap, buf, lane);
                 __syncwarp();
                 float z[32];
                 read_row(buf, lane, z);

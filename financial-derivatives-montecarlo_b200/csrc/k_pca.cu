@@ -127,45 +127,27 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 
 // Normals of points 32h..32h+31 for dimension `dim`, stored as fp16 at element e of the
 // 64-wide K-block of rows row0..row0+31 in the swizzled tile `A` (row r at r*128 bytes, 16-byte
-// chunk c at position c ^ (r & 7)).
+// chunk c at position c ^ (r & 7): the row bits of the transpose tile, so the strata walk's addresses
+// serve here too; row0 is a multiple of 32 and A starts at a multiple of kTileBytes).
+template <bool PARITY>
 __device__ __forceinline__ void sobol_tile_to_A(const uint32_t* __restrict__ dr, int D, int dim,
                                                 uint64_t h, float u_cap, unsigned char* A,
                                                 int row0, int e) {
-    const uint32_t* col = dr + dim;
-    const uint32_t L0 = __ldg(col), L1 = __ldg(col + D), L2 = __ldg(col + 2 * D),
-                   L3 = __ldg(col + 3 * D), L4 = __ldg(col + 4 * D);
-    uint32_t x = __ldg(col + 32 * D);
-    if (h & 1) x ^= L4;
-    uint32_t g = (uint32_t)(h ^ (h >> 1));
-    while (g) {
-        const int k = __ffs(g) - 1;
-        x ^= __ldg(col + (5 + k) * D);
-        g &= g - 1;
-    }
-    unsigned char* base = A + (e & 7) * 2;
-    const int chunk = e >> 3;
-    // four blocks of eight points (the gray-code steps as in sobol_tile), unrolled
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int r = row0 + 8 * b + i;
-            *reinterpret_cast<__half*>(base + r * 128 + ((chunk ^ (r & 7)) << 4)) =
-                __float2half_rn(sobol_normal(x, u_cap));
-            if (i < 7) {
-                x ^= gray_word8(i, L0, L1, L2);
-            } else if (b < 3) {
-                x ^= (b == 1) ? L4 : L3;
-            }
-        }
-    }
+    const uint32_t base = smem_u32(A + row0 * 128) ^ (uint32_t)(((e >> 3) << 4) | ((e & 7) * 2));
+    TileWalk w = tile_walk(dr, D, dim, h, base, nullptr, 0);
+    all_strata<PARITY>(
+        w, u_cap,
+        [](uint32_t a, float z) {
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(__half_as_ushort(__float2half_rn(z))) : "memory");
+        },
+        std::make_integer_sequence<int, 32>{});
 }
 
 template <class C>
 __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ KParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
-    unsigned char* sm = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
+    unsigned char* sm = smem_raw + ((0u - raw_addr) & (kTileBytes - 1));
     const int N = p.D;
     const int nkb = N >> 6;
     unsigned char* sB = sm;
@@ -240,7 +222,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
                 const uint64_t n = (p.g0 + (uint64_t)t * 4 + (uint64_t)quarter) * 32 + (uint64_t)lane;
                 C cons;
                 cons.init(p);
-                if constexpr (std::is_same<C, DumpC>::value) cons.bind(p, r, n);
+                if constexpr (is_dump<C>::value) cons.bind(p, r, n);
                 else cons.bind(r, n);
                 for (int c0 = 0; c0 < N; c0 += 32) {
                     float v[32];
@@ -270,7 +252,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
             const int j = item - r * p.items_per_rep;
             const int t_beg = j * p.gpi;
             const int t_end = min(t_beg + p.gpi, tiles_per_rep);
-            const uint32_t* dr = p.dirs + (size_t)r * 33 * (size_t)N;
+            const uint32_t* dr = p.dirs + (size_t)r * kDirRows * (size_t)N;
             for (int t = t_beg; t < t_end && !stop; t++, q++) {
                 const uint64_t h = p.g0 + (uint64_t)t * 4 + (uint64_t)rg;
                 for (int kb = 0; kb < nkb; kb++) {
@@ -281,7 +263,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
                         const bool ok = mbar_wait(smem_u32(&empty[s]), (uint32_t)(u - 1) & 1u);
                         if (!__all_sync(0xffffffffu, ok && !*s_fail)) { *s_fail = 1; stop = true; break; }
                     }
-                    sobol_tile_to_A(dr, N, kb * 64 + 32 * hf + lane, h, p.u_cap, sA + s * kAStageBytes, 32 * rg,
+                    sobol_tile_to_A<parity_of<C>::value>(dr, N, kb * 64 + 32 * hf + lane, h, p.u_cap, sA + s * kAStageBytes, 32 * rg,
                                     32 * hf + lane);
                     fence_proxy_async();   // generic-proxy stores visible to the tensor core's reads
                     mbar_arrive(smem_u32(&full[s]));
@@ -353,8 +335,11 @@ static const void* pca_payoff(int pay) {
     }
 }
 
-const void* lookup_pca(int model, int payoff, bool coupled, bool dump) {
-    if (dump) return (const void*)&k_pca<DumpC>;
+const void* lookup_pca_dump(bool parity) {
+    return parity ? (const void*)&k_pca<DumpC<true>> : (const void*)&k_pca<DumpC<false>>;
+}
+
+const void* lookup_pca(int model, int payoff, bool coupled) {
     if (coupled) {
         switch (model) {
             case MOD_GBM: return pca_payoff<MOD_GBM, true>(payoff);
@@ -370,7 +355,7 @@ const void* lookup_pca(int model, int payoff, bool coupled, bool dump) {
     }
 }
 
-size_t pca_smem_bytes(int N) { return (size_t)N * N * 2 + (size_t)kPcaStages * kAStageBytes + 256 + 1024; }
+size_t pca_smem_bytes(int N) { return (size_t)N * N * 2 + (size_t)kPcaStages * kAStageBytes + 256 + kTilePad; }
 int pca_threads() { return kPcaThreads; }
 int pca_warps() { return kPcaDrainWarps; }
 int pca_tile_paths() { return kPcaRows; }

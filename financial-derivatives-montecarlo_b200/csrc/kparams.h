@@ -47,6 +47,17 @@ constexpr int kAssistHelpers = 3;
 constexpr int kAssistTeam = 1 + kAssistHelpers;              // warps per owner
 constexpr int kAssistTeams = kWarpsPerBlock / kAssistTeam;   // owners per block
 constexpr int kAssistTeamBytes = kAssistSlots * 1024 * 4 + 2 * kAssistSlots * 8;
+// A transpose tile (32 x 32 floats) starts at a multiple of its size in the shared window; kTilePad is
+// what a launch adds to its dynamic shared memory for the alignment.
+constexpr int kTileBytes = 4096;
+constexpr int kTilePad = kTileBytes - 16;
+// Rows of a replica's direction table, D words each: rows 0-9 hold the pairs {R_k, row bits} of the
+// reduced basis (k = 0..4, pair k of dimension d at 2 (k D + d)), then W_5 .. W_31 and the digital shift, packed
+// (tile_walk, path_kernels.cuh).
+constexpr int kDirRowW5 = 10;
+constexpr int kDirRowShift = kDirRowW5 + 27;
+constexpr int kDirRows = kDirRowShift + 1;
+constexpr int kPlainRows = 33;   // rows of the plain table: words 0..31 and the shift
 
 struct KParams {
     // ---- geometry
@@ -96,9 +107,9 @@ struct KParams {
     float bbw[5][3];    // NOISE_BB_UNI: (wl, wr, sd) of window level u = 0..4
     // ---- PCA: M_pca (fp16, K-major rows = output step) device pointer
     const void* pca;
-    // ---- Sobol: pre-scrambled words, replica r at dirs + r * 33 * dstride, word k of dim d at
-    //      [k * dstride + d] (k = 32 is the digital shift); dstride >= D (the table may cover more
-    //      dimensions than this pass uses, as the book's per-level tables do)
+    // ---- Sobol: pre-scrambled words in reduced form, replica r at dirs + r * kDirRows * dstride (rows
+    //      of dstride words, kDirRows below); dstride >= D (the table may cover more dimensions than
+    //      this pass uses, as the book's per-level tables do)
     const uint32_t* dirs;
     int dstride;
     // ---- Philox

@@ -10,7 +10,7 @@
 //
 // Limits: at most kMaxDims Sobol dimensions (steps x factors), kMaxReplicas replicas and
 // kMaxItems work items; one-factor or Heston models without parameter arrays (GBM, Heston,
-// parametric Dupire), raw noise ordering.  The array costs kScratchBytes (about 2.7 MiB) on
+// parametric Dupire), raw noise ordering.  The array costs kScratchBytes (about 3.1 MiB) on
 // every GPU that loads the library, held until the process exits.
 //
 // Sharing: every call uses the same array and it keeps the last call's contents.  Nothing in
@@ -51,7 +51,7 @@ constexpr int kMaxReplicas = 32;
 constexpr int kMaxItems = 38912;
 static_assert(kMaxItems >= kTargetItems + kMaxReplicas, "partials sized for the engine's work split");
 constexpr size_t kTableBytes = (size_t)kMaxDims * 32 * sizeof(uint32_t);              // 64 KiB
-constexpr size_t kDirsBytes = (size_t)kMaxReplicas * 33 * kMaxDims * sizeof(uint32_t); // 2.06 MiB
+constexpr size_t kDirsBytes = (size_t)kMaxReplicas * kDirRows * kMaxDims * sizeof(uint32_t); // 2.4 MiB
 constexpr size_t kPartialBytes = (size_t)kMaxItems * 2 * sizeof(double);              // 608 KiB
 constexpr size_t kScratchBytes = kTableBytes + kDirsBytes + kPartialBytes;
 static_assert(kTableBytes % 256 == 0 && kDirsBytes % 256 == 0, "256-byte aligned sections");
@@ -150,9 +150,9 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
     const void* fn = (D <= 16) ? lookup_sobol_packed(k.model, p->kind, false) : nullptr;
     const bool packed = fn != nullptr;
     // the plain pass in the launch variant the autotuner keeps for these families on a B200 (it does
-    // not run here: no timing events on the caller's stream): the unrolled tile generator (all
-    // variants give the same bits)
-    if (!fn) fn = lookup_variant(GEN_SOBOL, NOISE_RAW, EST_PLAIN, k.model, p->kind, 2);
+    // not run here: no timing events on the caller's stream): four CTAs per SM (all variants give
+    // the same bits)
+    if (!fn) fn = lookup_variant(GEN_SOBOL, NOISE_RAW, EST_PLAIN, k.model, p->kind, 1);
     if (!fn) fn = lookup_pass(GEN_SOBOL, NOISE_RAW, EST_PLAIN, k.model, p->kind, 0);
     MCQ_REQUIRE(fn != nullptr, MCQ_ERR_UNSUPPORTED, "no fused kernel for this model / payoff");
     const uint64_t g0 = a.offset >> 5;
@@ -177,7 +177,7 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
     k.dirs = dirs;
     k.partials = partials;
 
-    size_t smem = (size_t)kWarpsPerBlock * 1024 * sizeof(float);
+    size_t smem = (size_t)kWarpsPerBlock * 1024 * sizeof(float) + kTilePad;
     int per_sm = 0;
     MCQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem));
     MCQ_REQUIRE(per_sm > 0, MCQ_ERR_INTERNAL, "kernel does not fit on an SM");

@@ -17,34 +17,28 @@
 // replica; warps take items round-robin.  Item boundaries depend only on the problem size, so
 // the result is bit-reproducible run to run.
 //
-// Sobol generation (warp-transposed).  For a tile of 32 dimensions, lane j owns dimension
-// d0 + j and produces its scrambled integers for all 32 points of the group by gray-code
-// recurrence: x(32h) = shift ^ XOR_{k in gray(h)} Lv[5+k] ^ [h odd] Lv[4], then
-// x(32h+i+1) = x(32h+i) ^ Lv[ctz(i+1)].  Lv are the direction words already multiplied by the
-// replica's Hong–Hickernell matrix (linearity of the scramble over F2), so each point costs
-// one XOR instead of 32 splitmix32 rows + 32 popcounts (hh_scramble, methods_cuda.cu:781-795).
-// The normals go through a 32x32 XOR-swizzled shared-memory transpose and come back one row
-// (one path) per lane.
+// Sobol generation (warp-transposed, in strata order).  For a tile of 32 dimensions, lane j owns
+// dimension d0 + j and produces its scrambled integers for all 32 points of the group: one XOR per
+// point with direction words already multiplied by the replica's Hong–Hickernell matrix (linearity of
+// the scramble over F2) instead of 32 splitmix32 rows + 32 popcounts (hh_scramble,
+// methods_cuda.cu:781-795).  Each dimension's 32 points of an aligned group fall into the 32 strata
+// [s/32, (s+1)/32) once each, so the lanes visit them stratum by stratum, all lanes in the same one at a
+// time: the inverse normal is then a polynomial with compile-time coefficients (inv_normal.cuh).  The
+// point a lane visits in a stratum is its own; its normal goes to that point's row of a 32x32
+// XOR-swizzled shared-memory tile and comes back one row (one path) per lane.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <type_traits>
+#include <utility>
 #include <cuda_fp16.h>
+#include "inv_normal.cuh"
 #include "kparams.h"
 
 namespace mcq {
 
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kTwoPow32Inv = 2.3283064365386963e-10f;   // 2^-32
 constexpr float kTwoPow24Inv = 5.9604644775390625e-08f;   // 2^-24
-
-// Direction word of the gray-code step from point i to point i + 1 inside a block of eight
-// (i = 0..6: word ctz(i + 1) = 0, 1, 0, 2, 0, 1, 0), written as bit tests of i so that an unrolled
-// i folds to one XOR operand.  (A recursive constexpr ctz called with the loop index is not
-// folded by the device compiler: it left ~10 integer and branch instructions per normal.)
-__device__ __forceinline__ uint32_t gray_word8(int i, uint32_t L0, uint32_t L1, uint32_t L2) {
-    return (i & 1) == 0 ? L0 : ((i & 2) ? L2 : L1);
-}
 
 // ------------------------------------------------------------------ hashing / scrambling
 
@@ -70,21 +64,24 @@ __device__ __forceinline__ uint32_t hh_linear(uint32_t v, uint32_t base) {
     return out;
 }
 
-// u = ((float)s + 1) * 2^-32 as in methods_cuda.cu:823; u_cap is 1.0f in reference-compat
-// mode (u may be 1 -> +inf) and 1 - 2^-24 otherwise.
-// ((float)x + 1) * 2^-32 == fma((float)x, 2^-32, 2^-32) bit for bit: scaling by a power of two
-// is exact, so both round the same real number once.
-__device__ __forceinline__ float sobol_normal(uint32_t x, float u_cap) {
-    const float u = fmaf((float)x, kTwoPow32Inv, kTwoPow32Inv);
-    return normcdfinvf(fminf(u, u_cap));
-}
-
 // ------------------------------------------------------------------ transpose buffer
 
 // 32 x 32 floats per warp, 16-byte chunks XOR-swizzled by row so that column writes
-// (lane = column) and float4 row reads (lane = row) are both bank-conflict free.
+// (lane = column) and float4 row reads (lane = row) are both bank-conflict free.  A tile starts at a
+// multiple of 4096 bytes of the shared window (kTileBytes; tile_base), so that the byte offset of (row,
+// col) is the XOR of row_bits(row) and 4 col and can be walked by XORs alone.
 __device__ __forceinline__ int swz(int row, int col) {
     return row * 32 + ((((col >> 2) ^ (row & 7)) << 2) | (col & 3));
+}
+
+__host__ __device__ __forceinline__ constexpr uint32_t row_bits(uint32_t row) {
+    return (row << 7) ^ ((row & 7u) << 4);
+}
+
+// The first tile of a kernel's dynamic shared memory: launches add kTilePad to what they use.
+__device__ __forceinline__ float* tile_base(void* smem) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
+    return reinterpret_cast<float*>(static_cast<char*>(smem) + ((0u - a) & (kTileBytes - 1)));
 }
 
 __device__ __forceinline__ void read_row(const float* buf, int lane, float (&z)[32]) {
@@ -96,37 +93,99 @@ __device__ __forceinline__ void read_row(const float* buf, int lane, float (&z)[
     }
 }
 
-// Lane owns dimension `dim` of replica table `dr` (words [k * D + dim]); writes the normals of
-// points 32h .. 32h+31 into column `lane` of the transpose buffer.
+// The 32 points of an aligned group are x = X ^ (combination of the five words L0..L4), their top five
+// bits taking every value once (the scramble is lower, the Sobol matrix upper triangular with unit
+// diagonals, so the leading 5 x 5 block of their product is invertible).  k_prescramble therefore
+// stores, per dimension, the basis in reduced form: R_k, the combination whose top five bits are bit k
+// alone, with the row offset of its points (row_bits of the point index), and every other word and
+// the digital shift reduced to zero top bits, where the row of that word goes instead.  A packed word
+// is so the group's point of stratum 0: x (top bits zero) and its row, both walked by the same XORs.
 //
-// The start word x(32h) = shift ^ XOR of v_k over the set bits k of gray(32h), and
-// gray(32h) = gray(h) << 5 | (h & 1) << 4, so a tile walks popcount(gray(h)) words from the
-// digital shift.  A caller that generates the same dimension for groups h - 1, h, h + 1, ... in
-// order keeps the start word of each tile in `slot` (shared memory) and passes cont = 1 from the
-// second group on: x(32h) = x(32(h - 1)) ^ v_4 ^ v_{5 + ctz(h)}, two words instead of the walk and
-// its chain of dependent loads (the same word, so the same normals).  cont = 2: the slot already
-// holds x(32h) (a tile generated again for the same group, as the adjoint's reverse sweep does).
-//
-// The 32 points run as four blocks of eight: inside a block the gray-code step is fixed (word
-// ctz(i + 1), gray_word8), between blocks (points 8, 16, 24) it XORs word 3 + ctz(b + 1).  UNR
-// blocks are unrolled at a time (1, 2 or 4): a larger unroll drops the loop's overhead but
-// multiplies the inlined inverse-normal code the instruction cache must hold; the fused pass
-// families are compiled with more than one and the autotuner picks (the same normals).
-__device__ __forceinline__ void sobol_block8(uint32_t& x, int b, uint32_t L0, uint32_t L1, uint32_t L2,
-                                             uint32_t L3, uint32_t L4, float u_cap, float* buf, int lane) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        buf[swz(8 * b + i, lane)] = sobol_normal(x, u_cap);
-        if (i < 7) x ^= gray_word8(i, L0, L1, L2);
-        else if (b < 3) x ^= (b == 1) ? L4 : L3;
+// Packed start word of group h: shift ^ W_{5+k} over the set bits k of gray(h), and, for odd h,
+// the row 31 that bit 4 of gray(32h) contributes.  A caller that generates the same dimension for groups
+// h - 1, h, h + 1, ... in order keeps the packed word of each tile in `slot` (shared memory) and passes
+// cont = 1 from the second group on: one word instead of the walk and its chain of dependent loads.
+// cont = 2: the slot already holds group h's word (a tile generated again for the same group, as the
+// adjoint's reverse sweep does).
+struct TileWalk {
+    uint32_t x, a;          // point and shared-memory address of the current stratum
+    uint2 R0, R1, R2, R3, R4;   // .x: R_k, .y: row_bits of its row
+};
+
+__device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
+                                              uint32_t base, uint32_t* slot, int cont) {
+    const uint2* rk = reinterpret_cast<const uint2*>(dr) + dim;
+    TileWalk w;
+    w.R0 = __ldg(rk);
+    w.R1 = __ldg(rk + D);
+    w.R2 = __ldg(rk + 2 * D);
+    w.R3 = __ldg(rk + 3 * D);
+    w.R4 = __ldg(rk + 4 * D);
+    const uint32_t* col = dr + dim;
+    uint32_t s;
+    if (slot != nullptr && cont == 2) {
+        s = *slot;
+    } else if (slot != nullptr && cont) {
+        s = *slot ^ 0xF8000000u ^ __ldg(col + (kDirRowW5 - 1 + __ffsll((long long)h)) * D);
+    } else {
+        s = __ldg(col + kDirRowShift * D) ^ (0u - ((uint32_t)h & 1u) & 0xF8000000u);
+        uint32_t g = (uint32_t)(h ^ (h >> 1));
+        while (g) {
+            s ^= __ldg(col + (kDirRowW5 - 1 + __ffs(g)) * D);
+            g &= g - 1;
+        }
     }
+    if (slot != nullptr) *slot = s;
+    w.x = s & 0x07FFFFFFu;
+    w.a = base ^ row_bits(s >> 27);
+    return w;
 }
 
-template <int UNR = 1>
-__device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int D, int dim,
-                                           bool active, uint64_t h, float u_cap, float* buf,
-                                           int lane, uint32_t* slot = nullptr, int cont = 0) {
-    static_assert(UNR == 1 || UNR == 2 || UNR == 4, "blocks unrolled: 1, 2 or 4");
+// Visits the strata in gray-code order 0, 1, 3, 2, ...: one step per template index.
+template <int T, bool PARITY, class STORE>
+__device__ __forceinline__ void stratum_step(TileWalk& w, float u_cap, const STORE& store) {
+    if constexpr (T > 0) {
+        constexpr int k = (T & 1) ? 0 : (T & 2) ? 1 : (T & 4) ? 2 : (T & 8) ? 3 : 4;
+        const uint2 R = k == 0 ? w.R0 : k == 1 ? w.R1 : k == 2 ? w.R2 : k == 3 ? w.R3 : w.R4;
+        w.x ^= R.x;
+        w.a ^= R.y;
+    }
+    if constexpr (PARITY) store(w.a, sobol_normal(w.x, u_cap));
+    else store(w.a, stratum_normal<T ^ (T >> 1)>(w.x, u_cap));
+}
+template <bool PARITY, class STORE, int... T>
+__device__ __forceinline__ void all_strata(TileWalk& w, float u_cap, const STORE& store,
+                                           std::integer_sequence<int, T...>) {
+    (stratum_step<T, PARITY>(w, u_cap, store), ...);
+}
+
+// Lane owns dimension `dim` of replica table `dr` (kDirRows rows of D words); writes the normals of
+// points 32h .. 32h+31 into column `lane` of the transpose tile.  PARITY: every normal from
+// normcdfinvf, the bits of the reference's generator (the exports); the priced passes take the
+// strata's polynomials.
+template <bool PARITY = false>
+__device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int D, int dim, bool active, uint64_t h,
+                                           float u_cap, float* buf, int lane, uint32_t* slot = nullptr,
+                                           int cont = 0) {
+    if (!active) return;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(buf) ^ ((uint32_t)lane << 2);
+    TileWalk w = tile_walk(dr, D, dim, h, base, slot, cont);
+    all_strata<PARITY>(
+        w, u_cap,
+        [](uint32_t a, float z) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(z) : "memory"); },
+        std::make_integer_sequence<int, 32>{});
+}
+
+// The generator's plain form, for the estimators whose outputs turn on single paths (the book's digital
+// deltas, the adjoint's node vegas): points in order and every normal from normcdfinvf, from the plain
+// table of 33 rows (words 0..31, shift).  Lane j's start word x(32h) = shift ^ XOR of v_k over the set
+// bits k of gray(32h), gray(32h) = gray(h) << 5 | (h & 1) << 4, then x(32h+i+1) = x(32h+i) ^
+// v_{ctz(i+1)}; slot and cont as in tile_walk (x(32h) = x(32(h - 1)) ^ v_4 ^ v_{5 + ctz(h)}).  The four
+// blocks of eight points are rolled: unrolled, the inlined inverse normal fills the instruction
+// cache of these kernels (book 641 -> 602 options/s).
+__device__ __forceinline__ void sobol_tile_plain(const uint32_t* __restrict__ dr, int D, int dim, bool active,
+                                                 uint64_t h, float u_cap, float* buf, int lane,
+                                                 uint32_t* slot = nullptr, int cont = 0) {
     if (!active) return;
     const uint32_t* col = dr + dim;
     const uint32_t L0 = __ldg(col), L1 = __ldg(col + D), L2 = __ldg(col + 2 * D),
@@ -141,21 +200,21 @@ __device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int 
         if (h & 1) x ^= L4;
         uint32_t g = (uint32_t)(h ^ (h >> 1));
         while (g) {
-            const int k = __ffs(g) - 1;
-            x ^= __ldg(col + (5 + k) * D);
+            x ^= __ldg(col + (4 + __ffs(g)) * D);
             g &= g - 1;
         }
     }
     if (slot != nullptr) *slot = x;
-    if constexpr (UNR == 4) {
-#pragma unroll
-        for (int b = 0; b < 4; b++) sobol_block8(x, b, L0, L1, L2, L3, L4, u_cap, buf, lane);
-    } else if constexpr (UNR == 2) {
-#pragma unroll 2
-        for (int b = 0; b < 4; b++) sobol_block8(x, b, L0, L1, L2, L3, L4, u_cap, buf, lane);
-    } else {
 #pragma unroll 1
-        for (int b = 0; b < 4; b++) sobol_block8(x, b, L0, L1, L2, L3, L4, u_cap, buf, lane);
+    for (int b = 0; b < 4; b++) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            buf[swz(8 * b + i, lane)] = sobol_normal(x, u_cap);
+            // word ctz(i + 1) as bit tests of i, which fold (a recursive constexpr ctz of the loop
+            // index does not)
+            if (i < 7) x ^= (i & 1) == 0 ? L0 : ((i & 2) ? L2 : L1);
+            else if (b < 3) x ^= (b == 1) ? L4 : L3;
+        }
     }
 }
 
@@ -747,7 +806,9 @@ struct BasketC {
 };
 
 // Parity probe: records the normals (raw) or increments (bridge) the pass consumed for one
-// path, so tests can compare the fused generation bit for bit with the reference stream.
+// path, so tests can compare the fused generation with the reference stream: bit for bit with PARITY
+// (the generator's normcdfinvf form), to the last places with the normals the priced passes use.
+template <bool PARITY>
 struct DumpC {
     __device__ __forceinline__ void flush() {}
     static constexpr int NST = 1;
@@ -993,28 +1054,40 @@ struct smem_tile_of { static constexpr bool value = false; };
 template <class C>
 struct smem_tile_of<C, std::void_t<decltype(C::SMEM_TILE)>> { static constexpr bool value = C::SMEM_TILE; };
 
-// One 32-path group h of a consumer.  `carry` (nullptr: none) holds the Sobol start words of
+template <class C>
+struct parity_of { static constexpr bool value = false; };
+template <>
+struct parity_of<DumpC<true>> { static constexpr bool value = true; };
+template <class C>
+struct is_dump { static constexpr bool value = false; };
+template <bool PARITY>
+struct is_dump<DumpC<PARITY>> { static constexpr bool value = true; };
+
+// One 32-path group h of a consumer (PLAIN: raw ordering through the generator's plain form).  `carry` (nullptr: none) holds the Sobol start words of
 // every tile the group generates, slot 32 t + lane for its t-th tile; cont says that the slots
 // hold group h - 1's words of the same replica (see sobol_tile).
-template <int GEN, int NOISE, class C, int GU = 1>
+template <int GEN, int NOISE, class C, bool PLAIN = false>
 __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint32_t* dr,
                                           uint32_t stream, uint64_t h, uint64_t n, float* buf,
                                           float* skel, int lane, uint32_t* carry = nullptr,
                                           bool cont = false) {
     const int D = p.D;
+    constexpr bool PARITY = parity_of<C>::value;
     if constexpr (NOISE == NOISE_RAW) {
         for (int d0 = 0; d0 < D; d0 += 32) {
             float z[32];
             uint32_t* slot = carry ? carry + d0 + lane : nullptr;
-            if constexpr (GEN == GEN_SOBOL && smem_tile_of<C>::value) {
-                sobol_tile<GU>(dr, p.dstride, d0 + lane, d0 + lane < D, h, p.u_cap, buf, lane, slot, cont);
+            if constexpr (GEN == GEN_SOBOL) {
+                if constexpr (PLAIN)
+                    sobol_tile_plain(dr, p.dstride, d0 + lane, d0 + lane < D, h, p.u_cap, buf, lane, slot, cont);
+                else
+                    sobol_tile<PARITY>(dr, p.dstride, d0 + lane, d0 + lane < D, h, p.u_cap, buf, lane, slot, cont);
                 __syncwarp();
-                cons.tile_smem(p, buf, lane, min(32, D - d0));
-                __syncwarp();
-                continue;
-            } else if constexpr (GEN == GEN_SOBOL) {
-                sobol_tile<GU>(dr, p.dstride, d0 + lane, d0 + lane < D, h, p.u_cap, buf, lane, slot, cont);
-                __syncwarp();
+                if constexpr (smem_tile_of<C>::value) {
+                    cons.tile_smem(p, buf, lane, min(32, D - d0));
+                    __syncwarp();
+                    continue;
+                }
                 read_row(buf, lane, z);
                 __syncwarp();
             } else {
@@ -1026,7 +1099,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
         // N <= 32 (one tile): dW_i = sum_k M[i][k] z_k with z and M rounded to fp16 as the
         // reference's cast + GEMM (methods_cuda.cu:1228-1229); larger N runs in k_pca.
         const int N = D;
-        sobol_tile<GU>(dr, p.dstride, lane, lane < N, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
+        sobol_tile<PARITY>(dr, p.dstride, lane, lane < N, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
         __syncwarp();
         float z[32];
         read_row(buf, lane, z);
@@ -1061,7 +1134,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
         const int N = D;
         if (N <= 32) {
             // one tile: the literal table-driven bridge (bb_apply, utils.cpp:104-124)
-            sobol_tile<GU>(dr, p.dstride, lane, lane < N, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
+            sobol_tile<PARITY>(dr, p.dstride, lane, lane < N, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
             __syncwarp();
             float z[32];
             read_row(buf, lane, z);
@@ -1089,7 +1162,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
             // carry slots: the skeleton tiles first, then one per window
             const int ns = (S + 31) & ~31;
             for (int t0 = 0; t0 < S; t0 += 32) {
-                sobol_tile<GU>(dr, p.dstride, t0 + lane, t0 + lane < S, h, p.u_cap, buf, lane,
+                sobol_tile<PARITY>(dr, p.dstride, t0 + lane, t0 + lane < S, h, p.u_cap, buf, lane,
                            carry ? carry + t0 + lane : nullptr, cont);
                 __syncwarp();
                 float z[32];
@@ -1114,7 +1187,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
                     const int u = 31 - __clz(lane + 1);
                     dim = (S << u) + (q << u) + (lane + 1 - (1 << u));
                 }
-                sobol_tile<GU>(dr, p.dstride, dim, act, h, p.u_cap, buf, lane,
+                sobol_tile<PARITY>(dr, p.dstride, dim, act, h, p.u_cap, buf, lane,
                            carry ? carry + ns + 32 * q + lane : nullptr, cont);
                 __syncwarp();
                 float z[32];
@@ -1160,8 +1233,10 @@ template <int GEN, class C>
 __device__ __forceinline__ void assisted_pass(const KParams& p, unsigned char* smem) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int team = wib / kAssistTeam, role = wib - team * kAssistTeam;   // role 0 owns the paths
-    float* ring = reinterpret_cast<float*>(smem + team * kAssistTeamBytes);
-    uint64_t* full = reinterpret_cast<uint64_t*>(ring + kAssistSlots * 1024);
+    // the teams' tiles first (each at a multiple of kTileBytes), then their mbarriers
+    float* tiles = tile_base(smem);
+    float* ring = tiles + team * kAssistSlots * 1024;
+    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + kAssistTeams * kAssistSlots * 1024) + team * 2 * kAssistSlots;
     uint64_t* empty = full + kAssistSlots;
     if (lane == 0 && role == 0) {
         for (int s = 0; s < kAssistSlots; s++) {
@@ -1209,7 +1284,7 @@ __device__ __forceinline__ void assisted_pass(const KParams& p, unsigned char* s
             }
             if (!stop) acc.flush(p.partials + (size_t)item * C::NST, lane);
         } else {
-            const uint32_t* dr = (GEN == GEN_SOBOL) ? p.dirs + (size_t)r * 33 * (size_t)p.dstride : nullptr;
+            const uint32_t* dr = (GEN == GEN_SOBOL) ? p.dirs + (size_t)r * kDirRows * (size_t)p.dstride : nullptr;
             const uint32_t stream = p.stream_base + (uint32_t)r;
             for (uint64_t h = gb; h < ge && !stop; h++) {
                 for (int t = 0; t < T; t++, u++) {
@@ -1249,7 +1324,7 @@ struct warp_acc_of { static constexpr bool value = false; };
 template <int MOD, int NB>
 struct warp_acc_of<BasketLevelC<MOD, NB>> { static constexpr bool value = true; };
 
-template <int GEN, int NOISE, class C, int MINB = 0, int GU = 1>
+template <int GEN, int NOISE, class C, int MINB = 0>
 __global__ void __launch_bounds__(kThreads, MINB ? MINB : (noise_is_bb(NOISE) ? 2 : kMinBlocks))
     k_pass(const __grid_constant__ KParams p) {
     extern __shared__ float4 smem4[];
@@ -1261,10 +1336,12 @@ __global__ void __launch_bounds__(kThreads, MINB ? MINB : (noise_is_bb(NOISE) ? 
     constexpr bool WACC = warp_acc_of<C>::value;
     const int skel_floats = (noise_is_bb(NOISE) && p.D > 32) ? ((p.D >> 5) + 1) * 32 : 0;
     const int acc_floats = WACC ? ((2 * C::NST + 3) & ~3) : 0;
-    float* buf = reinterpret_cast<float*>(smem4) + wib * (1024 + skel_floats + acc_floats + p.carry);
-    float* skel = buf + 1024;
-    double* wrec = reinterpret_cast<double*>(buf + 1024 + skel_floats);
-    uint32_t* carry = p.carry ? reinterpret_cast<uint32_t*>(buf + 1024 + skel_floats + acc_floats) : nullptr;
+    // the warps' transpose tiles, then per warp the bridge skeleton, the FP64 record and the carried words
+    float* tiles = tile_base(smem4);
+    float* buf = tiles + wib * 1024;
+    float* skel = tiles + kWarpsPerBlock * 1024 + wib * (skel_floats + acc_floats + p.carry);
+    double* wrec = reinterpret_cast<double*>(skel + skel_floats);
+    uint32_t* carry = p.carry ? reinterpret_cast<uint32_t*>(skel + skel_floats + acc_floats) : nullptr;
     const int total_warps = gridDim.x * kWarpsPerBlock;
     const uint64_t gend_all = p.g0 + p.G;
     for (int item = blockIdx.x * kWarpsPerBlock + wib; item < p.n_items; item += total_warps) {
@@ -1272,7 +1349,7 @@ __global__ void __launch_bounds__(kThreads, MINB ? MINB : (noise_is_bb(NOISE) ? 
         const int j = item - r * p.items_per_rep;
         const uint64_t gb = p.g0 + (uint64_t)j * (uint64_t)p.gpi;
         const uint64_t ge = min(gb + (uint64_t)p.gpi, gend_all);
-        const uint32_t* dr = (GEN == GEN_SOBOL) ? p.dirs + (size_t)r * 33 * (size_t)p.dstride : nullptr;
+        const uint32_t* dr = (GEN == GEN_SOBOL) ? p.dirs + (size_t)r * kDirRows * (size_t)p.dstride : nullptr;
         const uint32_t stream = p.stream_base + (uint32_t)r;
         Acc<WACC ? 1 : C::NST> acc;
         AccWarp<C::NST> wacc;
@@ -1310,9 +1387,9 @@ __global__ void __launch_bounds__(kThreads, MINB ? MINB : (noise_is_bb(NOISE) ? 
                 const uint64_t n = h * 32 + (uint64_t)lane;
                 C cons;
                 cons.init(p);
-                if constexpr (std::is_same<C, DumpC>::value) cons.bind(p, r, n);
+                if constexpr (is_dump<C>::value) cons.bind(p, r, n);
                 else cons.bind(r, n);
-                run_group<GEN, NOISE, C, GU>(p, cons, dr, stream, h, n, buf, skel, lane, carry, h != gb);
+                run_group<GEN, NOISE, C>(p, cons, dr, stream, h, n, buf, skel, lane, carry, h != gb);
                 float y[C::NST];
                 cons.finish(p, y);
                 const bool valid = n >= p.offset && n < p.offset + p.n_points;

@@ -6,7 +6,8 @@
 
 namespace mcq {
 
-const void* lookup_pca(int model, int payoff, bool coupled, bool dump);   // nullptr: unsupported
+const void* lookup_pca(int model, int payoff, bool coupled);   // nullptr: unsupported
+const void* lookup_pca_dump(bool parity);                       // the dump probe
 size_t pca_smem_bytes(int N);   // dynamic shared memory of a launch
 int pca_threads();      // block size
 int pca_warps();        // per-warp records per work item

@@ -37,9 +37,9 @@ constexpr long long kBatchFloats = 1LL << 27;   // Z: 256 MB fp16, dW: 512 MB fp
 __global__ void __launch_bounds__(kThreads) k_pca_normals(const uint32_t* __restrict__ dr, int N, uint64_t g0,
                                                          uint64_t G, uint64_t offset, uint64_t n_points,
                                                          float u_cap, __half* __restrict__ Z, int ldz) {
-    __shared__ float tile[kWarpsPerBlock][1024];
+    __shared__ float4 smem4[(kWarpsPerBlock * kTileBytes + kTilePad) / 16];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    float* buf = tile[wib];
+    float* buf = tile_base(smem4) + wib * 1024;
     const int ntiles = (N + 31) >> 5;
     const uint64_t tasks = G * (uint64_t)ntiles;
     for (uint64_t t = (uint64_t)blockIdx.x * kWarpsPerBlock + wib; t < tasks;
@@ -91,15 +91,7 @@ void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* 
     cublasHandle_t blas = static_cast<cublasHandle_t>(ws.blas.h);
     cublas_check(cublasSetStream(blas, ws.stream), "set stream");
 
-    if (!(ws.dirs_salt0 == a.salt0 && ws.dirs_R == R && ws.dirs_D == N)) {
-        uint32_t* d = (uint32_t*)ws.dirs.ensure(sizeof(uint32_t) * (size_t)R * 33 * N);
-        launch_prescramble(E.d_dv, a.salt0, R, N, d, ws.stream);
-        E.launches++;
-        ws.dirs_salt0 = a.salt0;
-        ws.dirs_R = R;
-        ws.dirs_D = N;
-    }
-    const uint32_t* dirs = (const uint32_t*)ws.dirs.p;
+    const uint32_t* dirs = direction_table(ws, a.salt0, R, N, false);
     const uint64_t pb = std::max<uint64_t>(32, (uint64_t)(kBatchFloats / N) / 32 * 32);
     const uint64_t pfirst = std::min<uint64_t>(pb, (a.n_points + 31) / 32 * 32);
     __half* Z = (__half*)ws.pca_z.ensure(sizeof(__half) * (size_t)pfirst * N);
@@ -110,7 +102,7 @@ void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* 
     KernelInfo& ki = kernel_info(fn, csmem);
     const float one = 1.0f, zero = 0.0f;
     for (int r = 0; r < R; r++) {
-        const uint32_t* dr = dirs + (size_t)r * 33 * N;
+        const uint32_t* dr = dirs + (size_t)r * kDirRows * N;
         for (uint64_t o = a.offset; o < a.offset + a.n_points; o += pb) {
             const uint64_t nb = std::min<uint64_t>(pb, a.offset + a.n_points - o);
             const int ld = (int)((nb + 31) / 32 * 32);

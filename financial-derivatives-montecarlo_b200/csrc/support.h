@@ -5,8 +5,12 @@
 
 namespace mcq {
 
+// the passes' direction table: [R][kDirRows][D] words (kparams.h)
 void launch_prescramble(const uint32_t* dv, uint32_t salt0, int R, int D, uint32_t* out,
                         cudaStream_t s);
+// the plain scrambled words and shift, [R][kPlainRows][D]
+void launch_prescramble_plain(const uint32_t* dv, uint32_t salt0, int R, int D, uint32_t* out,
+                              cudaStream_t s);
 void launch_finalize(const double* partials, int R, int ipr, int nstat, double* out,
                      cudaStream_t s);
 // one warp waits `polls` times on an mbarrier nothing arrives on, then records MCQ_ERR_TIMEOUT

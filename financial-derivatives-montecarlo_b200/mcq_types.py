@@ -15,6 +15,7 @@ FLAG_COMPAT_U_INF = 1
 FLAG_COMPAT_HESTON_MLMC = 2
 FLAG_HESTON_MILSTEIN = 8
 FLAG_BASKET_OWN_S0 = 16
+FLAG_DUMP_PRICED = 32
 
 _pd = C.POINTER(C.c_double)
 

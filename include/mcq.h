@@ -74,6 +74,9 @@ extern "C" {
                                            default: asset 0's S0 for every asset, as the
                                            reference (c_p.S0 = S0[0], methods_cuda.cu:1046, :538-542) */
 
+#define MCQ_FLAG_DUMP_PRICED        32  /* mcq_debug_pass_dump only: the normals as the priced passes
+                                           form them (default: the reference kernel's bits) */
+
 /* ---------------------------------------------------------------- parameter structs */
 typedef struct mcq_model {
     int32_t kind;                 /* MCQ_MODEL_* */
@@ -341,7 +344,7 @@ int mcq_is_pass(const mcq_model* m, const mcq_payoff* p, int n_steps, double z_s
  * the reference.  For callers that may not call cudaMalloc: code living in a process whose GPU
  * memory belongs to another allocator (a framework's caching allocator, a plugin host with a
  * fixed budget) and latency-critical paths where cudaMalloc / cudaFree would synchronise the
- * device.  Its scratch is one fixed __device__ array inside the library (about 2.7 MiB, held on
+ * device.  Its scratch is one fixed __device__ array inside the library (about 3.1 MiB, held on
  * every GPU that loads the library until exit); sums_device ([R][2] doubles) is the caller's.
  * Limits: GBM, Heston or parametric Dupire, raw ordering, n_steps x factors <= 512, R <= 32;
  * larger requests fail with MCQ_ERR_RANGE.  Same kernel family, work split and carried Sobol
@@ -358,7 +361,9 @@ int mcq_qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_steps, u
 /* ---------------------------------------------------------------- parity / debug exports
  * Hong–Hickernell scrambled Sobol stream (methods_cuda.cu:753-825): out[d * n + i] for
  * dimension dim0 + d and point index offset + i.  _u32 returns the scrambled integers,
- * _normal the N(0,1) values the path kernels consume. */
+ * _normal their N(0,1) values with the reference's bits (normcdfinvf).  The priced passes take
+ * the same u through one polynomial per 1/32 of the unit interval (the two end strata through
+ * normcdfinvf): the same normals to their last places, no further from the exact quantile. */
 int mcq_sobol_hh_u32(uint32_t salt, int dim0, int nd, uint32_t offset, int64_t n,
                      uint32_t* out_host);
 int mcq_sobol_hh_normal(uint32_t salt, int dim0, int nd, uint32_t offset, int64_t n,
@@ -372,8 +377,10 @@ int mcq_philox4x32_10(const uint32_t ctr[4], const uint32_t key[2], uint32_t out
 /* BB / PCA tables as the device sees them (for parity tests). */
 int mcq_bb_tables(mcq_handle bb, int* map_idx, float* wl, float* wr, float* sd);  /* per dimension */
 int mcq_pca_matrix(mcq_handle pca, float* M_colmajor_f32);
-/* The normals (raw) or time-ordered increments (bridge, PCA) that one fused pass consumed,
-   for bit-level parity tests: out_host[R][n_points][n_steps * d_noise].  n_points <= 2^20.
+/* The normals (raw) or time-ordered increments (bridge, PCA) of one fused pass:
+   out_host[R][n_points][n_steps * d_noise].  n_points <= 2^20.  The default form carries the
+   reference's bits (mcq_sobol_hh_normal) through the pass's generation, ordering and transposition;
+   with MCQ_FLAG_DUMP_PRICED in `flags` the normals are those that the priced passes consume.
    `bb` is the BB handle for MCQ_NOISE_BB and the PCA handle for MCQ_NOISE_PCA. */
 int mcq_debug_pass_dump(const mcq_model* m, int n_steps, int noise_mode, mcq_handle bb,
                         int use_sobol, uint32_t seed, uint32_t salt_base, int R, uint32_t offset,
