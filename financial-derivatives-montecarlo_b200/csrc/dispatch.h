@@ -21,6 +21,9 @@ const void* lookup_philox_plain(int model, int payoff);
 const void* lookup_philox_coupled(int model, int payoff);
 // est in {EST_CV_ASIAN, EST_CV_DUPIRE, EST_IS}, basket models (nb = 4, 8, 16)
 const void* lookup_misc(int gen, int noise, int est, int model, int nb);
+// single-level Sobol passes of baskets of n <= 16 assets, by exact width
+const void* lookup_basket_multi(int n);
+const void* lookup_basket_gbm(int n);
 // dump probes: the normals in normcdfinvf's bits (parity) or as the priced passes form them
 const void* lookup_dump(int gen, int noise, bool parity);
 

@@ -289,6 +289,14 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
         float* d = (float*)ws.aux.ensure(pk.size() * sizeof(float));
         MCQ_CUDA(cudaMemcpyAsync(d, pk.data(), pk.size() * sizeof(float), cudaMemcpyHostToDevice, ws.stream));
         k.bsk = d;
+        if (n <= kMaxBasket) {
+            for (int i = 0; i < n; i++) {
+                k.bkS0[i] = pk[i];
+                k.bkV[i] = pk[n + i];
+                k.bkW[i] = pk[2 * n + i];
+                for (int j = 0; j <= i; j++) k.bkL[i * (i + 1) / 2 + j] = pk[3 * n + i * n + j];
+            }
+        }
     }
     if (m.kind == MCQ_MODEL_LOCALVOL_GRID) {
         double K0, iK, t0, it;
@@ -537,7 +545,9 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     k.carry = 0;
     if (a.gen == GEN_SOBOL && !assist && !packed && gpi >= 2) {
         int tiles = 0;
-        if (a.noise == NOISE_RAW) tiles = (D + 31) / 32;
+        // a basket's tiles hold whole steps (BasketTileC)
+        const int td = (a.est == EST_PLAIN && !a.dump && nb > 0 && nb <= kMaxBasket) ? 32 / nb * nb : 32;
+        if (a.noise == NOISE_RAW) tiles = (D + td - 1) / td;
         else if ((a.noise == NOISE_BB || a.noise == NOISE_BB_UNI) && D > 32) tiles = ((D >> 5) + 31) / 32 + (D >> 5);
         else if (a.noise == NOISE_BB || a.noise == NOISE_BB_UNI || knoise == NOISE_PCA) tiles = 1;
         const size_t with = smem + (size_t)kWarpsPerBlock * 32 * tiles * sizeof(uint32_t);

@@ -20,17 +20,19 @@ static const void* misc_gen(int noise, int est, int model, int nb) {
         return nullptr;
     }
     if (model == MOD_MULTI) {
-        if (nb <= 4) return (const void*)&k_pass<GEN, NOISE_RAW, BasketC<MOD_MULTI, 4>>;
-        if (nb <= 8) return (const void*)&k_pass<GEN, NOISE_RAW, BasketC<MOD_MULTI, 8>>;
-        if (nb <= 16) return (const void*)&k_pass<GEN, NOISE_RAW, BasketC<MOD_MULTI, 16>>;
+        if (GEN == GEN_SOBOL && nb <= kMaxBasket) return lookup_basket_multi(nb);
+        if (nb <= 4) return (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, BasketC<MOD_MULTI, 4>>;
+        if (nb <= 8) return (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, BasketC<MOD_MULTI, 8>>;
+        if (nb <= 16) return (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, BasketC<MOD_MULTI, 16>>;
         if (nb <= kMaxWideBasket) return (const void*)&k_pass<GEN, NOISE_RAW, BasketWideC<MOD_MULTI>>;
         if (nb <= kMaxHugeBasket) return (const void*)&k_pass<GEN, NOISE_RAW, BasketWideC<MOD_MULTI, kMaxHugeBasket>>;
         return nullptr;
     }
     if (model == MOD_BASKET) {
-        if (nb <= 4) return (const void*)&k_pass<GEN, NOISE_RAW, BasketC<MOD_BASKET, 4>>;
-        if (nb <= 8) return (const void*)&k_pass<GEN, NOISE_RAW, BasketC<MOD_BASKET, 8>>;
-        if (nb <= 16) return (const void*)&k_pass<GEN, NOISE_RAW, BasketC<MOD_BASKET, 16>>;
+        if (GEN == GEN_SOBOL && nb <= kMaxBasket) return lookup_basket_gbm(nb);
+        if (nb <= 4) return (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, BasketC<MOD_BASKET, 4>>;
+        if (nb <= 8) return (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, BasketC<MOD_BASKET, 8>>;
+        if (nb <= 16) return (const void*)&k_pass<GEN_PHILOX, NOISE_RAW, BasketC<MOD_BASKET, 16>>;
         if (nb <= kMaxWideBasket) return (const void*)&k_pass<GEN, NOISE_RAW, BasketWideC<MOD_BASKET>>;
         if (nb <= kMaxHugeBasket) return (const void*)&k_pass<GEN, NOISE_RAW, BasketWideC<MOD_BASKET, kMaxHugeBasket>>;
         return nullptr;

@@ -95,6 +95,9 @@ struct KParams {
     int n_assets;
     int uncorrelated;
     const float* bsk;
+    // the same for baskets of at most kMaxBasket assets, in the parameter block (constant-bank operands):
+    // S0, second block (sigma or inverse S0), weights, and the lower triangle of L by rows
+    float bkS0[kMaxBasket], bkV[kMaxBasket], bkW[kMaxBasket], bkL[kMaxBasket * (kMaxBasket + 1) / 2];
     // ---- local-vol grid sigma[j * nK + i], uniform axes
     const float* lv;
     const float2* lv_rows;   // [n_steps + 1] time rows of the fine steps (lv_time_row)
