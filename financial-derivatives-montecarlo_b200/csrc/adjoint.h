@@ -4,9 +4,11 @@
 
 namespace mcq {
 
-// variant: the checkpoint interval (0: 16 steps, 1: 32, 2: 8; Heston has one)
-const void* lookup_adjoint(int model, int payoff, int variant);
-size_t adjoint_smem_bytes(int model, int n_steps, int n_nodes, int variant);
-int adjoint_variants(int model);
+const void* lookup_adjoint(int model, int payoff);
+int adjoint_warps(int model);   // per CTA
+int adjoint_node_copies_log2(int model, int n_steps, int n_nodes);   // KParams::node_copies_log2
+size_t adjoint_smem_bytes(int model, int n_steps, int n_nodes);
+// device scratch of one warp's 32 paths (KParams::path_scratch)
+size_t adjoint_path_bytes(int model, int n_steps);
 
 }  // namespace mcq

@@ -328,11 +328,10 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
 // ------------------------------------------------------------------ launcher
 
 
-// Resident blocks per SM of kernel `fn` at `smem` bytes of dynamic shared memory (kThreads
-// threads).  A kernel's dynamic shared-memory limit is raised to the device's opt-in maximum
+// Resident blocks per SM of kernel `fn` at `smem` bytes of dynamic shared memory.  A kernel's dynamic shared-memory limit is raised to the device's opt-in maximum
 // once, so that occupancy can be asked for several sizes (with and without carry slots) and any
 // of them launched.
-KernelInfo& kernel_info(const void* fn, size_t smem) {
+KernelInfo& kernel_info(const void* fn, size_t smem, int threads) {
     Engine& E = engine();
     const auto key = std::make_pair(fn, smem);
     auto it = E.kinfo.find(key);
@@ -344,7 +343,7 @@ KernelInfo& kernel_info(const void* fn, size_t smem) {
     }
     KernelInfo ki;
     ki.smem = smem;
-    MCQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ki.blocks_per_sm, fn, kThreads, smem));
+    MCQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ki.blocks_per_sm, fn, threads, smem));
     MCQ_REQUIRE(ki.blocks_per_sm > 0, MCQ_ERR_INTERNAL, "kernel does not fit on an SM");
     return E.kinfo[key] = ki;
 }
@@ -686,14 +685,7 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
     fill_params(ws, a, k);
     const int n_nodes = (m.kind == MCQ_MODEL_LOCALVOL_GRID) ? m.lv_nK * m.lv_nt : 0;
     MCQ_REQUIRE(n_nodes <= 4096, MCQ_ERR_UNSUPPORTED, "adjoint Greeks: at most 4096 grid nodes");
-    // the checkpoint interval is a launch variant (same bits); variants whose shared memory does
-    // not fit one CTA per SM are left out
-    int nvar = adjoint_variants(k.model);
-    while (nvar > 1 && adjoint_smem_bytes(k.model, n_steps, n_nodes, nvar - 1) > 227 * 1024) nvar--;
-    TuneState* trial = nullptr;
-    const uint64_t key = (1ULL << 40) | ((uint64_t)k.model << 4) | (uint64_t)p.kind;
-    const int variant = tune_pick(key, nvar, (double)R * (double)n_points * (double)n_steps, (double)(1 << 26), &trial);
-    const void* fn = lookup_adjoint(k.model, p.kind, variant);
+    const void* fn = lookup_adjoint(k.model, p.kind);
     MCQ_REQUIRE(fn != nullptr, MCQ_ERR_UNSUPPORTED, "no adjoint kernel for this model / payoff");
     const uint64_t g0 = offset >> 5;
     const uint64_t G = ((offset + n_points - 1) >> 5) - g0 + 1;
@@ -712,16 +704,27 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
         MCQ_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(double) * n_nodes, ws.stream));
     }
     k.node_out = d_nodes;
-    const size_t smem = adjoint_smem_bytes(k.model, n_steps, n_nodes, variant);
-    KernelInfo& ki = kernel_info(fn, smem);
-    long long blocks = std::min<long long>(((long long)k.n_items + kWarpsPerBlock - 1) / kWarpsPerBlock,
-                                           (long long)ki.blocks_per_sm * E.sm_count);
-    blocks = std::max<long long>(blocks, 1);
+    const size_t smem = adjoint_smem_bytes(k.model, n_steps, n_nodes);
+    k.node_copies_log2 = adjoint_node_copies_log2(k.model, n_steps, n_nodes);
+    const int warps = adjoint_warps(k.model);
+    KernelInfo& ki = kernel_info(fn, smem, warps * 32);
+    // items are dealt to the CTAs in turn, one warp of each first
+    long long blocks = std::min<long long>((long long)k.n_items, (long long)ki.blocks_per_sm * E.sm_count);
+    // the path scratch: two stretches per resident warp (930 MB at 512 steps on a full GPU); where so much is
+    // not to be had, fewer CTAs share the work
+    const size_t per_block = (size_t)warps * adjoint_path_bytes(k.model, n_steps);
+    for (;;) {
+        try {
+            k.path_scratch = (float4*)ws.paths.ensure((size_t)blocks * per_block);
+            break;
+        } catch (const Error&) {
+            if (blocks == 1) throw;
+            blocks = (blocks + 1) / 2;
+        }
+    }
     double* d_out = (double*)ws.sums.ensure(sizeof(double) * (size_t)R * 4);
     void* args[] = {&k};
-    if (trial) MCQ_CUDA(cudaEventRecord(trial->ev[variant][0], ws.stream));
-    MCQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(kThreads), args, smem, ws.stream));
-    if (trial) MCQ_CUDA(cudaEventRecord(trial->ev[variant][1], ws.stream));
+    MCQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3((unsigned)(warps * 32)), args, smem, ws.stream));
     launch_finalize(k.partials, R, k.items_per_rep, 4, d_out, ws.stream);
     E.launches += 2;
     MCQ_CUDA(cudaGetLastError());
@@ -747,7 +750,7 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
     out.n_paths = (int64_t)R * (int64_t)n_points;
     out.n_nodes = n_nodes;
     out.launches = E.launches - l0;
-    out.path_steps = 3.0 * (double)out.n_paths * n_steps;   // forward + recompute + reverse
+    out.path_steps = 3.0 * (double)out.n_paths * n_steps;   // forward, path read back, reverse
     if (node_vega)
         for (int i = 0; i < n_nodes; i++) node_vega[i] = nv[i] / (double)out.n_paths;
     out.time_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

@@ -63,6 +63,7 @@ struct Workspace {
     PinnedBuf hsums, haux;
     DevBuf xbuf[8];       // long-lived scratch of the batched book (book.cu): kept across calls
     PinnedBuf xpin[2];
+    DevBuf paths;         // the adjoint's path scratch
     DevBuf pca_z, pca_dw, pca_tmp;   // the large-N PCA route (pca_large.cu): fp16 normals, increments
     struct Blas {                    // its cuBLAS handle, created on first use
         void* h = nullptr;
@@ -162,8 +163,8 @@ struct PassArgs {
 // B200 at four CTAs per SM: a warp's last item then costs at most an eighth of the pass (with
 // three per warp the small first passes of the adaptive drivers lost up to a quarter).
 inline constexpr long long kTargetItems = 148LL * 32 * 8;
-// the adjoint's split: about eight items per resident warp (two CTAs of eight warps per SM)
-inline constexpr long long kTargetItemsAdjoint = 148LL * 16 * 8;
+// the adjoint's split: one item per resident warp (24 an SM), whose waiting paths pass from group to group
+inline constexpr long long kTargetItemsAdjoint = 148LL * 24;
 
 int noise_dim(const mcq_model& m);
 // KParams for a pass (make_params); basket / local-vol arrays are uploaded into ws.aux.
@@ -190,7 +191,7 @@ void join_caller_stream(Workspace& ws, cudaStream_t caller);
 // an unread status of an earlier asynchronous pass).
 int* arm_err_word(Workspace& ws);
 // Occupancy / shared-memory set-up of a kernel for a dynamic shared-memory size (cached).
-KernelInfo& kernel_info(const void* fn, size_t smem);
+KernelInfo& kernel_info(const void* fn, size_t smem, int threads = kThreads);
 // Pathwise adjoint Greeks over R scrambled replicas (k_adjoint.cu).
 void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t salt_base, int R,
                  uint64_t offset, uint64_t n_points, int flags, mcq_greeks& out, double* node_vega);

@@ -123,6 +123,8 @@ struct KParams {
     float* dump;
     // ---- adjoint: per-node local-vol sensitivities, summed over paths (FP64)
     double* node_out;
+    int node_copies_log2;   // copies of the node array in a CTA's shared memory
+    float4* path_scratch;   // every step's state and normals, one stretch per resident warp (k_adjoint.cu)
     // ---- bounded-wait / error reporting
     int* err;
     // ---- NOISE_DW: increment i of point offset + row at dw_in[i * dw_stride + row]

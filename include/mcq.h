@@ -164,7 +164,7 @@ typedef struct mcq_greeks {
     int32_t n_nodes;                              /* grid nodes written to node_vega (0 otherwise) */
     int32_t launches;
     double  time_s;
-    double  path_steps;                           /* forward + recompute + reverse path-steps */
+    double  path_steps;                           /* three sweeps: forward, path read back, reverse */
 } mcq_greeks;
 
 /* One option of a batched book (mcq_book_price), priced by MLQMC to its own eps.  Either
@@ -273,7 +273,8 @@ int mcq_run_is(const mcq_model* gbm, const mcq_payoff* european, double z_star, 
  * step with MCQ_FLAG_HESTON_MILSTEIN); node_vega (optional, lv_nt * lv_nK doubles, same layout
  * as lv_sigma) receives dV/dsigma(K_i, t_j).  Lipschitz payoffs only: European, arithmetic Asian,
  * lookback.  n_steps: multiple of 32 in [32, 1024] (Heston: of 16 in [16, 1024]); path states
- * are checkpointed every 16 steps and recomputed in the reverse sweep. */
+ * go through a scratch array in device memory (up to 256 bytes a step for each resident warp, 512 for
+ * Heston; kept until mcq_shutdown). */
 int mcq_adjoint(const mcq_model* m, const mcq_payoff* p, int n_steps, uint32_t salt_base, int R,
                 uint32_t offset, int64_t n_points, int flags, mcq_greeks* out, double* node_vega);
 
