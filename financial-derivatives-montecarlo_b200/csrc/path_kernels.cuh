@@ -34,11 +34,11 @@
 #include <cuda_fp16.h>
 #include "inv_normal.cuh"
 #include "kparams.h"
+#include "philox.cuh"
 
 namespace mcq {
 
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kTwoPow24Inv = 5.9604644775390625e-08f;   // 2^-24
 
 // ------------------------------------------------------------------ hashing / scrambling
 
@@ -215,42 +215,6 @@ __device__ __forceinline__ void sobol_tile_plain(const uint32_t* __restrict__ dr
             if (i < 7) x ^= (i & 1) == 0 ? L0 : ((i & 2) ? L2 : L1);
             else if (b < 3) x ^= (b == 1) ? L4 : L3;
         }
-    }
-}
-
-// ------------------------------------------------------------------ Philox4x32-10
-
-__device__ __forceinline__ uint4 philox10(uint4 c, uint2 k) {
-#pragma unroll
-    for (int r = 0; r < 10; r++) {
-        if (r) { k.x += 0x9E3779B9u; k.y += 0xBB67AE85u; }
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-        c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
-    }
-    return c;
-}
-
-__device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, float& z0, float& z1) {
-    const float u1 = ((float)(a >> 8) + 0.5f) * kTwoPow24Inv;
-    const float u2 = ((float)(b >> 8) + 0.5f) * kTwoPow24Inv;
-    const float rr = sqrtf(-2.0f * logf(u1));
-    float s, c;
-    sincospif(2.0f * u2, &s, &c);
-    z0 = rr * s;
-    z1 = rr * c;
-}
-
-// Normals 32t .. 32t+31 of path `path` on stream `stream` (block b = dims 4b..4b+3).
-__device__ __forceinline__ void philox_tile(uint32_t seed, uint32_t stream, uint64_t path, int t,
-                                            float (&z)[32]) {
-    const uint2 key = make_uint2(seed, 0x6D637121u);
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const uint4 o = philox10(make_uint4((uint32_t)(8 * t + q), (uint32_t)path,
-                                            (uint32_t)(path >> 32), stream), key);
-        box_muller(o.x, o.y, z[4 * q], z[4 * q + 1]);
-        box_muller(o.z, o.w, z[4 * q + 2], z[4 * q + 3]);
     }
 }
 

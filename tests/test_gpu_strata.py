@@ -40,3 +40,18 @@ def test_priced_normals_of_carried_groups(gpu, model, n_steps, R, n, offset):
     for r in range(R):
         ref = gpu.sobol_hh_normal(11 + r, 0, n_steps * gpu.noise_dim(m), offset, n).T.astype(np.float64)
         assert (np.abs(dump[r] - ref) <= (TOL_INNER + TOL_END) * np.abs(ref)).all()
+
+
+@pytest.mark.parametrize("model,n_steps", [("gbm", 1), ("gbm", 33), ("heston", 50)])
+@pytest.mark.parametrize("first", [0, 1000, (1 << 32) - 20])
+def test_counter_based_normals_vs_fp64(gpu, orc, model, n_steps, first):
+    """Box-Muller on Philox words: an ulp each from the logarithm's fit and rounding (halved by the root), the root,
+    the sine or cosine and the product: below 4 x 2^-23 relative, plus the sine's 2^-23 2^-23 at its zeros."""
+    m = gpu.gbm() if model == "gbm" else gpu.heston()
+    D, n = n_steps * gpu.noise_dim(m), 40
+    dump = gpu.debug_pass_dump(m, n_steps, gpu.RAW, use_sobol=False, seed=9, salt_base=3, R=2, offset=first & 0xffffffff,
+                               n_points=n)
+    for r in range(2):
+        for i in range(n):
+            ref = orc.philox_normals(9, 3 + r, (first & 0xffffffff) + i, D)
+            assert (np.abs(dump[r, i] - ref) <= 4 * 2.0 ** -23 * np.abs(ref) + 2.0 ** -44).all(), (r, i)
