@@ -185,7 +185,7 @@ void run_mlmc(const mcq_model& m, const mcq_payoff& p, double eps, const mcq_mlm
     int L = 2;
     std::vector<double> E(max_L + 1, 0.0), V(max_L + 1, 0.0);
     std::vector<long long> N(max_L + 1, 0);
-    std::vector<double*> dsum(max_L + 1, nullptr);
+    std::vector<double*> hsum(max_L + 1, nullptr);
     double ps = 0.0;
     uint32_t seed_ctr = 0;   // one fresh Philox stream per launch (the reference: seed 42, 43, ...)
 
@@ -203,18 +203,15 @@ void run_mlmc(const mcq_model& m, const mcq_payoff& p, double eps, const mcq_mlm
         a.m = &m; a.p = &p; a.n_steps = (int)nf; a.est = EST_COUPLED; a.M = M; a.level0 = (l == 0);
         a.mlmc_h = true; a.gen = GEN_PHILOX; a.R = 1; a.offset = 0; a.n_points = (uint64_t)n;
         a.seed = cfg.seed; a.stream0 = seed_ctr++; a.flags = cfg.flags;
-        dsum[l] = (double*)w.sums.ensure((size_t)nstat_of(EST_COUPLED, m.kind) * sizeof(double));
-        pass_async(w, a, dsum[l]);
+        hsum[l] = pass_to_host(w, a);
         ps += (double)n * (double)(nf + (l ? nf / M : 0));
     };
     // collect_level (:1400-1409)
     auto collect = [&](int l) -> std::vector<double> {
         Workspace& w = engine().ws(1 + l);
-        double* h = (double*)w.hsums.ensure(4 * sizeof(double));
-        MCQ_CUDA(cudaMemcpyAsync(h, dsum[l], 4 * sizeof(double), cudaMemcpyDeviceToHost, w.stream));   // first 4 stats
         MCQ_CUDA(cudaStreamSynchronize(w.stream));
         check_err_word(w);
-        return std::vector<double>(h, h + 4);
+        return std::vector<double>(hsum[l], hsum[l] + 4);   // first 4 stats
     };
 
     for (int l = 0; l <= L; l++) launch(l, cfg.pilot_n);   // :1412-1421
@@ -304,7 +301,7 @@ void run_mlqmc(const mcq_model& m, const mcq_payoff& p, double eps, const mcq_ml
     int L = 2;
     std::vector<double> E(max_L + 1, 0.0), sig2(max_L + 1, 0.0);
     std::vector<long long> N(max_L + 1, 0), next_off(max_L + 1, 0);
-    std::vector<double*> dsum(max_L + 1, nullptr);
+    std::vector<double*> hsum(max_L + 1, nullptr);
     double ps = 0.0;
     auto nfine = [&](int l) -> long long {
         long long n = ml.n0_steps;
@@ -346,18 +343,16 @@ void run_mlqmc(const mcq_model& m, const mcq_payoff& p, double eps, const mcq_ml
         a.seed = qc.salt_base; a.stream0 = qc.salt_base + (uint32_t)(l * R);
         a.offset = (uint64_t)next_off[l];
         a.n_points = (uint64_t)n;
-        dsum[l] = (double*)w.sums.ensure((size_t)R * ns * sizeof(double));
-        pass_async(w, a, dsum[l]);
+        hsum[l] = pass_to_host(w, a);
         next_off[l] += n;
         ps += (double)R * (double)n * (double)(nf + (l ? nf / M : 0));
     };
     // collect_level (:1927-1944): mean and sample variance of the R replica means
     auto collect = [&](int l, long long n) -> std::pair<double, double> {
         Workspace& w = engine().ws(1 + l);
-        double* h = (double*)w.hsums.ensure((size_t)R * ns * sizeof(double));
-        MCQ_CUDA(cudaMemcpyAsync(h, dsum[l], (size_t)R * ns * sizeof(double), cudaMemcpyDeviceToHost, w.stream));
         MCQ_CUDA(cudaStreamSynchronize(w.stream));
         check_err_word(w);
+        const double* h = hsum[l];
         double mm = 0.0;
         for (int r = 0; r < R; r++) mm += h[ns * r] / n;
         mm /= R;

@@ -286,9 +286,12 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
         k.uncorrelated = unc ? 1 : 0;
         k.inv_S0 = 1.0f / (float)m.S0_vec[0];     // c_p.S0 = S0[0] (:1046)
         k.S0 = (float)m.S0_vec[0];
-        float* d = (float*)ws.aux.ensure(pk.size() * sizeof(float));
-        MCQ_CUDA(cudaMemcpyAsync(d, pk.data(), pk.size() * sizeof(float), cudaMemcpyHostToDevice, ws.stream));
-        k.bsk = d;
+        // the single-level Sobol passes of register-resident baskets read the parameter block only
+        if (n > kMaxBasket || a.gen != GEN_SOBOL || a.est != EST_PLAIN) {
+            float* d = (float*)ws.aux.ensure(pk.size() * sizeof(float));
+            MCQ_CUDA(cudaMemcpyAsync(d, pk.data(), pk.size() * sizeof(float), cudaMemcpyHostToDevice, ws.stream));
+            k.bsk = d;
+        }
         if (n <= kMaxBasket) {
             for (int i = 0; i < n; i++) {
                 k.bkS0[i] = pk[i];
@@ -310,7 +313,8 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
         const size_t grid_bytes = (nn * sizeof(float) + 15) & ~(size_t)15;
         const int n_rows = a.n_steps + 1;
         char* d = (char*)ws.aux.ensure(grid_bytes + (size_t)n_rows * sizeof(float2));
-        MCQ_CUDA(cudaMemcpyAsync(d, g.data(), nn * sizeof(float), cudaMemcpyHostToDevice, ws.stream));
+        if (nn > (size_t)kLvArgNodes)
+            MCQ_CUDA(cudaMemcpyAsync(d, g.data(), nn * sizeof(float), cudaMemcpyHostToDevice, ws.stream));
         k.lv = (const float*)d;
         k.lv_nK = m.lv_nK;
         k.lv_nt = m.lv_nt;
@@ -319,7 +323,7 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
         k.lv_t0 = (float)t0;
         k.lv_inv_dt = (float)it;
         float2* rows = (float2*)(d + grid_bytes);
-        launch_lv_rows(k, rows, n_rows, ws.stream);
+        launch_lv_rows(k, g.data(), (float*)d, (int)nn, rows, n_rows, ws.stream);
         engine().launches++;
         k.lv_rows = rows;
     }
@@ -414,6 +418,12 @@ const uint32_t* direction_table(Workspace& ws, uint32_t salt0, int R, int D, boo
     return (const uint32_t*)ws.dirs.p;
 }
 
+// PCA orderings that neither k_pass (N <= 32) nor the tensor-core pass (N in {64, 128, 256}) holds
+static bool pca_is_large(const PassArgs& a) {
+    const int D = a.n_steps * noise_dim(*a.m);
+    return a.noise == NOISE_PCA && D > 32 && D != 64 && D != 128 && D != 256 && !a.dump;
+}
+
 void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     Engine& E = engine();
     MCQ_REQUIRE(a.m && a.p, MCQ_ERR_INVALID, "null model or payoff");
@@ -458,7 +468,7 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     }
     // fused: N <= 32 inside k_pass, N in {64, 128, 256} in the tensor-core pass (its factor in
     // shared memory); other N through fp16 normals, a library GEMM and the pass on increments
-    if (a.noise == NOISE_PCA && D > 32 && D != 64 && D != 128 && D != 256 && !a.dump) {
+    if (pca_is_large(a)) {
         pca_large_pass_async(ws, a, k, d_out);
         return;
     }
@@ -566,7 +576,7 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     if (assist) k.err = arm_err_word(ws);
     void* args[] = {&k};
     if (trial) MCQ_CUDA(cudaEventRecord(trial->ev[variant][0], ws.stream));
-    MCQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(kThreads), args, smem, ws.stream));
+    MCQ_CUDA(launch_dependent(fn, (unsigned)blocks, kThreads, args, smem, ws.stream));
     if (trial) MCQ_CUDA(cudaEventRecord(trial->ev[variant][1], ws.stream));
     launch_finalize(k.partials, a.R, k.items_per_rep, nst, d_out, ws.stream);
     E.launches += 2;
@@ -614,41 +624,49 @@ void pca_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* d_out)
     long long blocks = std::min<long long>((long long)k.n_items, (long long)per_sm * E.sm_count);
     blocks = std::max<long long>(blocks, 1);
     void* args[] = {&k};
-    MCQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(pca_threads()), args, smem, ws.stream));
+    MCQ_CUDA(launch_dependent(fn, (unsigned)blocks, (unsigned)pca_threads(), args, smem, ws.stream));
     launch_finalize(k.partials, a.R, k.items_per_rep * pca_warps(), nst, d_out, ws.stream);
     E.launches += 2;
     MCQ_CUDA(cudaGetLastError());
 }
 
-// A bounded device wait that gave up leaves MCQ_ERR_TIMEOUT in the workspace's error word.  The
-// word is cleared only when it is armed afresh after a check, so a failure of an asynchronous pass
-// stays there until the next synchronous call on the workspace reads it.
+// A bounded device wait that gave up leaves MCQ_ERR_TIMEOUT in the workspace's error word, which is pinned
+// host memory.  The word is cleared only when it is armed afresh after a check, so a failure of an
+// asynchronous pass stays there until the next synchronous call on the workspace reads it.
 int* arm_err_word(Workspace& ws) {
     int* err = (int*)ws.err.ensure(sizeof(int));
     if (!ws.err_armed) {
-        MCQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ws.stream));
+        *(volatile int*)err = 0;
         ws.err_armed = true;
     }
     return err;
 }
 
+// After a synchronisation of the workspace stream, which a pass on a caller's stream has been joined into
+// (join_caller_stream): every pass that may have set the word has ended.
 void check_err_word(Workspace& ws) {
     if (!ws.err_armed) return;
-    // read on the workspace stream, which a pass on a caller's stream has been joined into
-    // (join_caller_stream), so the word is read after every pass that may have set it
-    int* h = (int*)ws.haux.ensure(sizeof(int));
-    MCQ_CUDA(cudaMemcpyAsync(h, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, ws.stream));
-    MCQ_CUDA(cudaStreamSynchronize(ws.stream));
+    const int code = *(volatile int*)ws.err.p;
     ws.err_armed = false;
-    MCQ_REQUIRE(*h == 0, MCQ_ERR_TIMEOUT, "a bounded device-side wait timed out (status " + std::to_string(*h) + ")");
+    MCQ_REQUIRE(code == 0, MCQ_ERR_TIMEOUT, "a bounded device-side wait timed out (status " + std::to_string(code) + ")");
+}
+
+double* pass_to_host(Workspace& ws, const PassArgs& a) {
+    const size_t n = (size_t)a.R * (a.dump ? 1 : nstat_of(a.est, a.m->kind));
+    double* h = (double*)ws.hsums.ensure(sizeof(double) * n);
+    if (a.n_points == 0 || pca_is_large(a)) {   // these add up or clear their sums in device memory
+        double* d = (double*)ws.sums.ensure(sizeof(double) * n);
+        pass_async(ws, a, d);
+        MCQ_CUDA(cudaMemcpyAsync(h, d, sizeof(double) * n, cudaMemcpyDeviceToHost, ws.stream));
+    } else {
+        pass_async(ws, a, h);
+    }
+    return h;
 }
 
 std::vector<double> pass_sync(Workspace& ws, const PassArgs& a) {
     const size_t n = (size_t)a.R * (a.dump ? 1 : nstat_of(a.est, a.m->kind));
-    double* d = (double*)ws.sums.ensure(sizeof(double) * n);
-    pass_async(ws, a, d);
-    double* h = (double*)ws.hsums.ensure(sizeof(double) * n);
-    MCQ_CUDA(cudaMemcpyAsync(h, d, sizeof(double) * n, cudaMemcpyDeviceToHost, ws.stream));
+    const double* h = pass_to_host(ws, a);
     MCQ_CUDA(cudaStreamSynchronize(ws.stream));
     check_err_word(ws);
     return std::vector<double>(h, h + n);
@@ -722,17 +740,17 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
             blocks = (blocks + 1) / 2;
         }
     }
-    double* d_out = (double*)ws.sums.ensure(sizeof(double) * (size_t)R * 4);
+    double* s = (double*)ws.hsums.ensure(sizeof(double) * (size_t)R * 4);   // pinned: written by the kernel
     void* args[] = {&k};
-    MCQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3((unsigned)(warps * 32)), args, smem, ws.stream));
-    launch_finalize(k.partials, R, k.items_per_rep, 4, d_out, ws.stream);
+    MCQ_CUDA(launch_dependent(fn, (unsigned)blocks, (unsigned)(warps * 32), args, smem, ws.stream));
+    launch_finalize(k.partials, R, k.items_per_rep, 4, s, ws.stream);
     E.launches += 2;
     MCQ_CUDA(cudaGetLastError());
-    std::vector<double> s((size_t)R * 4);
-    MCQ_CUDA(cudaMemcpyAsync(s.data(), d_out, sizeof(double) * s.size(), cudaMemcpyDeviceToHost, ws.stream));
-    std::vector<double> nv(n_nodes);
-    if (n_nodes)
-        MCQ_CUDA(cudaMemcpyAsync(nv.data(), d_nodes, sizeof(double) * n_nodes, cudaMemcpyDeviceToHost, ws.stream));
+    double* nv = nullptr;
+    if (n_nodes) {
+        nv = (double*)ws.haux.ensure(sizeof(double) * n_nodes);
+        MCQ_CUDA(cudaMemcpyAsync(nv, d_nodes, sizeof(double) * n_nodes, cudaMemcpyDeviceToHost, ws.stream));
+    }
     MCQ_CUDA(cudaStreamSynchronize(ws.stream));
     double mean[4] = {0, 0, 0, 0}, se[4] = {0, 0, 0, 0};
     for (int q = 0; q < 4; q++) {

@@ -58,9 +58,9 @@ struct PinnedBuf {
 struct Workspace {
     cudaStream_t stream = nullptr;
     cudaEvent_t joined = nullptr;
-    DevBuf partials, sums, dirs, aux, dump, err;
-    bool err_armed = false;   // err holds a fresh status from the last tensor-core pass
-    PinnedBuf hsums, haux;
+    DevBuf partials, sums, dirs, aux, dump;
+    bool err_armed = false;   // err holds a fresh status from the last tensor-core or assisted pass
+    PinnedBuf hsums, haux, err;
     DevBuf xbuf[8];       // long-lived scratch of the batched book (book.cu): kept across calls
     PinnedBuf xpin[2];
     DevBuf paths;         // the adjoint's path scratch
@@ -173,14 +173,18 @@ int nstat_of(int est);
 int nstat_of(int est, int model_kind);   // basket levels carry per-asset deltas
 // The direction table of a pass on ws.stream: the passes' reduced form, or the plain one (kparams.h).
 const uint32_t* direction_table(Workspace& ws, uint32_t salt0, int R, int D, bool plain);
-// Enqueue one pass on ws.stream; d_out receives [R][nstat] doubles (device).
+// Enqueue one pass on ws.stream; d_out receives [R][nstat] doubles (device; pinned host memory for all but
+// large PCA orderings and empty ranges).
 void pass_async(Workspace& ws, const PassArgs& a, double* d_out);
 // Tensor-core PCA pass (N in {64, 128, 256}); called by pass_async.
 void pca_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* d_out);
 // PCA orderings the tensor-core pass does not hold (N > 32 outside {64, 128, 256}): fp16 normals,
 // one library GEMM and the fused pass on the increments, batch by batch (pca_large.cu)
 void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* d_out);
-// Enqueue, copy back and wait; returns [R][nstat].
+// Enqueue one pass whose sums arrive in the workspace's pinned buffer ([R][nstat], readable after a
+// synchronisation of ws.stream).
+double* pass_to_host(Workspace& ws, const PassArgs& a);
+// Enqueue and wait; returns [R][nstat].
 std::vector<double> pass_sync(Workspace& ws, const PassArgs& a);
 // After a synchronisation of ws.stream: raises MCQ_ERR_TIMEOUT if a bounded device-side wait of
 // the workspace's last tensor-core or assisted pass gave up.

@@ -116,6 +116,7 @@ __device__ __forceinline__ float4 path_load(const float4* p) { return __ldcs(p);
 template <int MOD, int PAY>
 __global__ void __launch_bounds__(kAdjThreads, 1) k_adjoint(const __grid_constant__ KParams p) {
     extern __shared__ float4 smem4[];
+    grid_dependency_wait();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int N = p.n_steps;
     float* buf = reinterpret_cast<float*>(smem4) + wib * 1024;       // 32 x 32 transpose tile
@@ -336,6 +337,7 @@ __device__ __forceinline__ void heston_adj_step(const KParams& p, float& S, floa
 template <int PAY>
 __global__ void __launch_bounds__(kThreads, 3) k_adjoint_heston(const __grid_constant__ KParams p) {
     extern __shared__ float4 smem4[];
+    grid_dependency_wait();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int N = p.n_steps, D = 2 * N, n_tiles = D / 32;
     float* buf = reinterpret_cast<float*>(smem4) + wib * 1024;   // 32 x 32 transpose tile

@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();   // the factor is the handle's; the direction words are the kernel before's
     const uint32_t tbase = *tslot;
 
     // Every role walks the same sequence: items blockIdx.x, + gridDim.x, ...; tiles [t_beg, t_end)
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
     __syncwarp();   // the issuer warp reconverges
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && *s_fail) atomicExch(p.err, MCQ_ERR_TIMEOUT_CODE);
+    if (tid == 0 && *s_fail) *(volatile int*)p.err = MCQ_ERR_TIMEOUT_CODE;
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(ncols));

@@ -1,7 +1,10 @@
 // k_support.cu — small kernels around the fused pass: per-replica direction-word scrambling,
 // the deterministic cross-item reduction, and the Sobol stream export used by parity tests.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include "path_kernels.cuh"
 #include "support.h"
 
@@ -78,23 +81,49 @@ __global__ void __launch_bounds__(1024) k_prescramble(const uint32_t* __restrict
     }
 }
 
-// out[r][s] = sum over j of partials[(r * ipr + j) * nstat + s]; fixed summation order.
-__global__ void k_finalize(const double* __restrict__ partials, int ipr, int nstat,
-                           double* __restrict__ out) {
-    __shared__ double red[256];
-    const int r = blockIdx.x, t = threadIdx.x;
-    for (int s = 0; s < nstat; s++) {
-        double v = 0.0;
-        for (int j = t; j < ipr; j += 256) v += partials[((size_t)r * ipr + j) * nstat + s];
-        red[t] = v;
-        __syncthreads();
-        for (int o = 128; o > 0; o >>= 1) {
-            if (t < o) red[t] += red[t + o];
-            __syncthreads();
-        }
-        if (t == 0) out[(size_t)r * nstat + s] = red[0];
-        __syncthreads();
+// out[r][s] = sum over j of partials[(r * ipr + j) * NST + s]; fixed summation order.  A cluster of CTAs per
+// replica, each over every n-th run of 256 records, its sums gathered through distributed shared memory:
+// with one CTA a pass of a single replica (plain Monte Carlo, 37,888 records) waited 25 us for it.
+// `out` may be host memory: the synchronous passes read their sums there after the stream's end, without a copy.
+constexpr int kFinThreads = 256;
+template <int NST>
+__global__ void __launch_bounds__(kFinThreads) k_finalize(const double* __restrict__ partials, int ipr,
+                                                          double* __restrict__ out) {
+    __shared__ double red[kFinThreads / 32][NST];
+    __shared__ double total[NST];
+    auto cluster = cooperative_groups::this_cluster();
+    const int nc = (int)cluster.num_blocks(), c = (int)cluster.block_rank(), r = blockIdx.x / nc;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double v[NST];
+#pragma unroll
+    for (int s = 0; s < NST; s++) v[s] = 0.0;
+    grid_dependency_wait();
+    const double* rec = partials + (size_t)r * ipr * NST;
+#pragma unroll 4
+    for (int j = c * kFinThreads + t; j < ipr; j += nc * kFinThreads) {
+#pragma unroll
+        for (int s = 0; s < NST; s++) v[s] += rec[(size_t)j * NST + s];
     }
+#pragma unroll
+    for (int s = 0; s < NST; s++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
+        if (lane == 0) red[warp][s] = v[s];
+    }
+    __syncthreads();
+    if (t < NST) {
+        double x = 0.0;
+        for (int w = 0; w < kFinThreads / 32; w++) x += red[w][t];
+        total[t] = x;
+    }
+    if (nc > 1) cluster.sync();
+    else __syncthreads();
+    if (c == 0 && t < NST) {
+        double x = 0.0;
+        for (int b = 0; b < nc; b++) x += *cluster.map_shared_rank(&total[t], b);
+        out[(size_t)r * NST + t] = x;
+    }
+    if (nc > 1) cluster.sync();   // the other CTAs' shared memory stays until it has been read
 }
 
 // Scrambled integers / normals of one replica by the direct gray-code form:
@@ -134,9 +163,36 @@ void launch_prescramble_plain(const uint32_t* dv, uint32_t salt0, int R, int D, 
     k_prescramble_plain<<<blocks, 256, 0, s>>>(dv, salt0, R, D, out);
 }
 
+// A launch whose CTAs may be placed while the stream's previous kernel drains; the kernel itself waits
+// for that kernel's results (grid_dependency_wait).
+cudaError_t launch_dependent(const void* fn, unsigned blocks, unsigned threads, void** args, size_t smem,
+                             cudaStream_t s, unsigned cluster) {
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 void launch_finalize(const double* partials, int R, int ipr, int nstat, double* out,
                      cudaStream_t s) {
-    k_finalize<<<R, 256, 0, s>>>(partials, ipr, nstat, out);
+    const void* fn = nstat == 1 ? (const void*)&k_finalize<1> : nstat == 2 ? (const void*)&k_finalize<2>
+                   : nstat == 4 ? (const void*)&k_finalize<4> : nstat == 7 ? (const void*)&k_finalize<7>
+                                                              : (const void*)&k_finalize<4 + kMaxBasket>;
+    // up to eight CTAs a replica, four records a thread
+    unsigned nc = 1;
+    while (nc < 8 && (long long)nc * kFinThreads * 4 < ipr) nc *= 2;
+    void* args[] = {&partials, &ipr, &out};
+    launch_dependent(fn, (unsigned)R * nc, kFinThreads, args, 0, s, nc);   // errors: cudaGetLastError at the caller
 }
 
 void launch_sobol_export(const uint32_t* tab, int D, int dim0, int nd, uint32_t offset,
@@ -158,21 +214,37 @@ __global__ void k_wait_probe(int* err, uint32_t polls) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(asst_addr(&bar)), "r"(1));
     __syncthreads();
     const bool ok = asst_wait(&bar, 0u, polls);
-    if (!__all_sync(0xffffffffu, ok) && threadIdx.x == 0) atomicExch(err, MCQ_ERR_TIMEOUT_CODE);
+    if (!__all_sync(0xffffffffu, ok) && threadIdx.x == 0) *(volatile int*)err = MCQ_ERR_TIMEOUT_CODE;
 }
 
 void launch_wait_probe(int* err, uint32_t polls, cudaStream_t s) {
     k_wait_probe<<<1, 32, 0, s>>>(err, polls);
 }
 
-// Time rows of the grid local-vol model for steps 0 .. n - 1 of a pass (lv_time_row).
-__global__ void k_lv_rows(const __grid_constant__ KParams p, float2* rows, int n) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        rows[k] = lv_time_row(p, k);
+// Time rows of the grid local-vol model for steps 0 .. n - 1 of a pass (lv_time_row).  Surfaces of up to
+// kLvArgNodes nodes come as a kernel argument and are written to `grid` on the way: no copy from
+// pageable host memory, which is staged before the call goes on.
+struct LvGrid { float g[kLvArgNodes]; };
+template <class G>
+__global__ void k_lv_rows(const __grid_constant__ KParams p, const __grid_constant__ G g, float* grid, int nodes,
+                          float2* rows, int n) {
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = i0; k < n; k += gridDim.x * blockDim.x) rows[k] = lv_time_row(p, k);
+    if constexpr (sizeof(G) > 1)
+        for (int i = i0; i < nodes; i += gridDim.x * blockDim.x) grid[i] = g.g[i];
 }
+struct NoGrid {};
 
-void launch_lv_rows(const KParams& p, float2* rows, int n, cudaStream_t s) {
-    k_lv_rows<<<(n + 255) / 256, 256, 0, s>>>(p, rows, n);
+void launch_lv_rows(const KParams& p, const float* host_grid, float* grid, int nodes, float2* rows, int n,
+                    cudaStream_t s) {
+    const int blocks = std::max(8, (n + 255) / 256);
+    if (nodes <= kLvArgNodes) {
+        LvGrid g;
+        std::memcpy(g.g, host_grid, sizeof(float) * (size_t)nodes);
+        k_lv_rows<<<blocks, 256, 0, s>>>(p, g, grid, nodes, rows, n);
+    } else {
+        k_lv_rows<<<blocks, 256, 0, s>>>(p, NoGrid{}, grid, nodes, rows, n);
+    }
 }
 
 }  // namespace mcq

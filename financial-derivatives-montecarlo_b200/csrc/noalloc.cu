@@ -203,7 +203,7 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
 
     launch_prescramble(table, salt_base, R, D, dirs, stream);
     void* args[] = {&k};
-    MCQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(kThreads), args, smem, stream));
+    MCQ_CUDA(launch_dependent(fn, (unsigned)blocks, kThreads, args, smem, stream));
     launch_finalize(partials, R, k.items_per_rep, 2, sums_device, stream);
     MCQ_CUDA(cudaGetLastError());
 }

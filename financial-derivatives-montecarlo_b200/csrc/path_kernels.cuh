@@ -40,6 +40,11 @@ namespace mcq {
 
 constexpr float kLog2e = 1.4426950408889634f;
 
+// Programmatic dependent launch (launch_dependent): wait for the kernel before; nothing without the launch
+// attribute.  No kernel lets its successor start early: pass CTAs placed beside the running prescramble
+// CTAs ended up unevenly over the SMs (Heston level 680 -> 714 us).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------ hashing / scrambling
 
 // splitmix32 (methods_cuda.cu:753-759).
@@ -1346,7 +1351,7 @@ __device__ __forceinline__ void assisted_pass(const KParams& p, unsigned char* s
             }
         }
     }
-    if (stop && lane == 0) atomicExch(p.err, MCQ_ERR_TIMEOUT_CODE);
+    if (stop && lane == 0) *(volatile int*)p.err = MCQ_ERR_TIMEOUT_CODE;
 }
 
 __host__ __device__ constexpr bool noise_is_bb(int noise) { return noise == NOISE_BB || noise == NOISE_BB_UNI; }
@@ -1363,6 +1368,7 @@ template <int GEN, int NOISE, class C, int MINB = 0>
 __global__ void __launch_bounds__(kThreads, MINB ? MINB : (noise_is_bb(NOISE) ? 2 : kMinBlocks))
     k_pass(const __grid_constant__ KParams p) {
     extern __shared__ float4 smem4[];
+    grid_dependency_wait();
     if constexpr (NOISE == NOISE_ASSIST) {
         assisted_pass<GEN, C>(p, reinterpret_cast<unsigned char*>(smem4));
         return;

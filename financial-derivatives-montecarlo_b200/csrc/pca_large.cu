@@ -98,7 +98,7 @@ void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* 
     float* dW = (float*)ws.pca_dw.ensure(sizeof(float) * (size_t)pfirst * N);
     double* tmp = (double*)ws.pca_tmp.ensure(sizeof(double) * nst);
     MCQ_CUDA(cudaMemsetAsync(d_out, 0, sizeof(double) * (size_t)R * nst, ws.stream));
-    const size_t csmem = (size_t)kWarpsPerBlock * 1024 * sizeof(float);
+    const size_t csmem = (size_t)kWarpsPerBlock * 1024 * sizeof(float) + kTilePad;
     KernelInfo& ki = kernel_info(fn, csmem);
     const float one = 1.0f, zero = 0.0f;
     for (int r = 0; r < R; r++) {
