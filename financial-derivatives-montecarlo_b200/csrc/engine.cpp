@@ -215,9 +215,13 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
     // FP32 ulps of 1, and rounding it there biases the mean reversion by up to 0.4 % at 2^18 steps
     // (the reference rounds expf(-kappa h) itself, methods_cuda.cu:282)
     k.om_f = (float)(-std::expm1(-(double)k.kappa * (double)h));
+    k.L10s = (float)((double)k.L10 * k.sqrt_h);
+    k.L11s = (float)((double)k.L11 * k.sqrt_h);
     k.sigma0 = (float)m.sigma0;
     k.alpha = (float)m.alpha;
     k.bm1 = (float)m.beta_d - 1.0f;
+    constexpr double kLog2E = 1.4426950408889634;
+    k.dup_f = (float)(-(double)k.alpha * kLog2E * h);
     if (m.kind == MCQ_MODEL_DUPIRE) k.sigma = k.sigma0;   // :1041 sigma_eff for the GBM control
 
     if (a.est == EST_COUPLED) {
@@ -225,6 +229,7 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
         k.n_coarse = a.level0 ? 0 : a.n_steps / a.M;
         k.hc = (float)(m.T / std::max(k.n_coarse, 1));
         k.om_c = (float)(-std::expm1(-(double)k.kappa * (double)k.hc));
+        k.dup_c = (float)(-(double)k.alpha * kLog2E * k.hc);
         if (a.level0) k.M = INT_MAX;   // the coarse path never steps on level 0
     }
     if (m.kind == MCQ_MODEL_HESTON && (a.flags & MCQ_FLAG_HESTON_MILSTEIN)) {
@@ -533,8 +538,11 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     k.g0 = g0;
     k.G = G;
 
+    // a basket's tiles hold whole steps (BasketTileC)
+    const int tile_dims = (a.est == EST_PLAIN && !a.dump && nb > 0 && nb <= kMaxBasket) ? 32 / nb * nb : 32;
     if (a.gen == GEN_SOBOL) {
-        k.dirs = direction_table(ws, a.salt0, a.R, D, false);
+        k.dstride = table_dims(D, tile_dims);
+        k.dirs = direction_table(ws, a.salt0, a.R, k.dstride, false);
     }
     const int nst = a.dump ? 1 : k.nstat;
     k.nstat = nst;
@@ -554,9 +562,7 @@ void pass_async(Workspace& ws, const PassArgs& a, double* d_out) {
     k.carry = 0;
     if (a.gen == GEN_SOBOL && !assist && !packed && gpi >= 2) {
         int tiles = 0;
-        // a basket's tiles hold whole steps (BasketTileC)
-        const int td = (a.est == EST_PLAIN && !a.dump && nb > 0 && nb <= kMaxBasket) ? 32 / nb * nb : 32;
-        if (a.noise == NOISE_RAW) tiles = (D + td - 1) / td;
+        if (a.noise == NOISE_RAW) tiles = (D + tile_dims - 1) / tile_dims;
         else if ((a.noise == NOISE_BB || a.noise == NOISE_BB_UNI) && D > 32) tiles = ((D >> 5) + 31) / 32 + (D >> 5);
         else if (a.noise == NOISE_BB || a.noise == NOISE_BB_UNI || knoise == NOISE_PCA) tiles = 1;
         const size_t with = smem + (size_t)kWarpsPerBlock * 32 * tiles * sizeof(uint32_t);

@@ -171,6 +171,8 @@ int noise_dim(const mcq_model& m);
 void fill_params(Workspace& ws, const PassArgs& a, KParams& k);
 int nstat_of(int est);
 int nstat_of(int est, int model_kind);   // basket levels carry per-asset deltas
+// Dimensions a pass's table covers: up to the last lane of its last tile.
+inline int table_dims(int D, int tile_dims) { return (D + tile_dims - 1) / tile_dims * tile_dims + (32 - tile_dims); }
 // The direction table of a pass on ws.stream: the passes' reduced form, or the plain one (kparams.h).
 const uint32_t* direction_table(Workspace& ws, uint32_t salt0, int R, int D, bool plain);
 // Enqueue one pass on ws.stream; d_out receives [R][nstat] doubles (device; pinned host memory for all but

@@ -82,6 +82,13 @@ struct StrataTable {
     };
 };
 
+// End strata: z = kEndSlope r + sum of k[i] (r - 3)^i.
+constexpr float kEndSlope = 0x1.2d6abep+0f;   // sqrt(2 ln 2)
+struct EndTable {
+    float k[10] = {-0x1.4b0e7ep-1f, 0x1.0d9b8ap-3f, -0x1.01e6p-5f, 0x1.075c9cp-7f, -0x1.1715aap-9f,
+                                0x1.3287dcp-11f, -0x1.6131eep-13f, 0x1.8170bep-15f, -0x1.2c50c2p-17f, 0x1.b4e718p-21f};
+};
+
 // |z| of the end strata from t = min(u, 1 - u) <= 1/32; t = 0 (u = 1 in reference-compat mode) gives
 // +inf: the leading coefficient and the linear term are positive.
 __device__ __forceinline__ float end_stratum(float t) {
@@ -89,17 +96,11 @@ __device__ __forceinline__ float end_stratum(float t) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(t));
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-l));
     const float d = r - 3.0f;
-    float p = 0x1.b4e718p-21f;
-    p = fmaf(p, d, -0x1.2c50c2p-17f);
-    p = fmaf(p, d, 0x1.8170bep-15f);
-    p = fmaf(p, d, -0x1.6131eep-13f);
-    p = fmaf(p, d, 0x1.3287dcp-11f);
-    p = fmaf(p, d, -0x1.1715aap-9f);
-    p = fmaf(p, d, 0x1.075c9cp-7f);
-    p = fmaf(p, d, -0x1.01e6p-5f);
-    p = fmaf(p, d, 0x1.0d9b8ap-3f);
-    p = fmaf(p, d, -0x1.4b0e7ep-1f);
-    return fmaf(0x1.2d6abep+0f, r, p);
+    constexpr EndTable e{};
+    float p = e.k[9];
+#pragma unroll
+    for (int i = 8; i >= 0; i--) p = fmaf(p, d, e.k[i]);
+    return fmaf(kEndSlope, r, p);
 }
 
 // The normal of x, whose top five bits are S.

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(1024) k_prescramble(const uint32_t* __restrict
         const uint32_t base = salt ^ (uint32_t)d;
         const uint32_t mask = lane == 0 ? 0u : 0xFFFFFFFFu << (32 - lane);
         const uint32_t mrow = (1u << (31 - lane)) | (splitmix32(base ^ (uint32_t)lane) & mask);
-        const uint32_t v = __ldg(dv + (size_t)d * 32 + lane);
+        const uint32_t v = __ldg(dv + (size_t)min(d, 19999) * 32 + lane);   // (beyond: lanes nobody reads)
         uint32_t w = 0;
 #pragma unroll
         for (int j = 0; j < 32; j++)

@@ -82,7 +82,9 @@ struct KParams {
     // ---- model (single precision, as the reference's c_p)
     float S0, inv_S0, mu, T, h, sqrt_h, sigma;
     float kappa, theta, xi, L10, L11, v0, om_f;    // om_f = 1 - exp(-kappa h), from expm1
+    float L10s, L11s;                              // L10, L11 times sqrt(h)
     float sigma0, alpha, bm1;                      // Dupire: bm1 = beta_d - 1
+    float dup_f, dup_c;                            // -alpha log2(e) times the fine / coarse step
     float hc, om_c;                                // coarse step, 1 - exp(-kappa hc)
     float mil;                                     // Heston Milstein: xi^2/4 (0: Euler)
     // ---- payoff

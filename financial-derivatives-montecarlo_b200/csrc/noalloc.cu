@@ -175,6 +175,7 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
     uint32_t* dirs = reinterpret_cast<uint32_t*>(base + kTableBytes);
     double* partials = reinterpret_cast<double*>(base + kTableBytes + kDirsBytes);
     k.dirs = dirs;
+    k.dstride = table_dims(D, 32);   // at most kMaxDims
     k.partials = partials;
 
     size_t smem = (size_t)kWarpsPerBlock * 1024 * sizeof(float) + kTilePad;
@@ -201,7 +202,7 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
     blocks = std::min<long long>(blocks, (long long)per_sm * sms);
     blocks = std::max<long long>(blocks, 1);
 
-    launch_prescramble(table, salt_base, R, D, dirs, stream);
+    launch_prescramble(table, salt_base, R, k.dstride, dirs, stream);
     void* args[] = {&k};
     MCQ_CUDA(launch_dependent(fn, (unsigned)blocks, kThreads, args, smem, stream));
     launch_finalize(partials, R, k.items_per_rep, 2, sums_device, stream);

@@ -82,7 +82,6 @@ __device__ __forceinline__ int swz(int row, int col) {
 __host__ __device__ __forceinline__ constexpr uint32_t row_bits(uint32_t row) {
     return (row << 7) ^ ((row & 7u) << 4);
 }
-
 // The first tile of a kernel's dynamic shared memory: launches add kTilePad to what they use.
 __device__ __forceinline__ float* tile_base(void* smem) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
@@ -114,8 +113,23 @@ __device__ __forceinline__ void read_row(const float* buf, int lane, float (&z)[
 // adjoint's reverse sweep does).
 struct TileWalk {
     uint32_t x, a;          // point and shared-memory address of the current stratum
-    uint2 R0, R1, R2, R3, R4;   // .x: R_k, .y: row_bits of its row
+    uint2 R0, R1, R2, R3, R4;   // .x: R_k, .y: the row bits of its row
 };
+
+// The packed word of group h's point of stratum 0 (slot and cont as above, without the store).
+__device__ __forceinline__ uint32_t start_word(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
+                                               const uint32_t* slot, int cont) {
+    const uint32_t* col = dr + dim;
+    if (slot != nullptr && cont == 2) return *slot;
+    if (slot != nullptr && cont) return *slot ^ 0xF8000000u ^ __ldg(col + (kDirRowW5 - 1 + __ffsll((long long)h)) * D);
+    uint32_t s = __ldg(col + kDirRowShift * D) ^ (0u - ((uint32_t)h & 1u) & 0xF8000000u);
+    uint32_t g = (uint32_t)(h ^ (h >> 1));
+    while (g) {
+        s ^= __ldg(col + (kDirRowW5 - 1 + __ffs(g)) * D);
+        g &= g - 1;
+    }
+    return s;
+}
 
 __device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
                                               uint32_t base, uint32_t* slot, int cont) {
@@ -126,20 +140,7 @@ __device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, i
     w.R2 = __ldg(rk + 2 * D);
     w.R3 = __ldg(rk + 3 * D);
     w.R4 = __ldg(rk + 4 * D);
-    const uint32_t* col = dr + dim;
-    uint32_t s;
-    if (slot != nullptr && cont == 2) {
-        s = *slot;
-    } else if (slot != nullptr && cont) {
-        s = *slot ^ 0xF8000000u ^ __ldg(col + (kDirRowW5 - 1 + __ffsll((long long)h)) * D);
-    } else {
-        s = __ldg(col + kDirRowShift * D) ^ (0u - ((uint32_t)h & 1u) & 0xF8000000u);
-        uint32_t g = (uint32_t)(h ^ (h >> 1));
-        while (g) {
-            s ^= __ldg(col + (kDirRowW5 - 1 + __ffs(g)) * D);
-            g &= g - 1;
-        }
-    }
+    const uint32_t s = start_word(dr, D, dim, h, slot, cont);
     if (slot != nullptr) *slot = s;
     w.x = s & 0x07FFFFFFu;
     w.a = base ^ row_bits(s >> 27);
@@ -167,12 +168,13 @@ __device__ __forceinline__ void all_strata(TileWalk& w, float u_cap, const STORE
 // Lane owns dimension `dim` of replica table `dr` (kDirRows rows of D words); writes the normals of
 // points 32h .. 32h+31 into column `lane` of the transpose tile.  PARITY: every normal from
 // normcdfinvf, the bits of the reference's generator (the exports); the priced passes take the
-// strata's polynomials.
+// strata's polynomials.  Every lane takes part, one beyond the path's dimensions
+// in a column nobody reads (the table covers whole tiles, table_dims): the branch around the tile cost 0.5 of 18.7
+// instructions per normal.
 template <bool PARITY = false>
-__device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int D, int dim, bool active, uint64_t h,
+__device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
                                            float u_cap, float* buf, int lane, uint32_t* slot = nullptr,
                                            int cont = 0) {
-    if (!active) return;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(buf) ^ ((uint32_t)lane << 2);
     TileWalk w = tile_walk(dr, D, dim, h, base, slot, cont);
     all_strata<PARITY>(
@@ -308,27 +310,29 @@ __device__ __forceinline__ float lv_sigma_row(const KParams& p, float S, float2 
     return fmaf(b, hi - lo, lo);
 }
 
-// sqrt(V+) of the Heston step with the hardware's approximate square root (`sqrt.approx.f32`,
+// sqrt(V+) of the Heston step with the hardware's approximate square root (`sqrt.approx.ftz.f32`,
 // relative error about 2^-23, exact at 0 and +inf) instead of the correctly rounded one, whose
 // refinement and special-case branch cost 9 % of a coupled Heston level pass.  The error scales
 // the diffusion coefficient of S and V by 1 +- 1e-7 and does not enter any drift, so it biases
-// neither the level means nor their differences.
+// neither the level means nor their differences.  (ftz: a variance below 2^-126 counts as 0; without
+// it each root carries a rescaling of such arguments.)
 __device__ __forceinline__ float sqrt_approx(float v) {
     float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
 
 // Parametric Dupire local volatility sigma0 e^{-alpha t} (S/S0)^(beta - 1) = sigma0 2^{(beta - 1) log2(S/S0)
-// - alpha t log2(e)}, x = S/S0, with the hardware's approximate base-2 logarithm and exponential
-// (`lg2.approx.f32`, `ex2.approx.f32`: errors about 2^-22, the same special values: log2 of 0 is
-// -inf, of a negative x NaN, 2^-inf = 0).  As with the Heston square root, the error scales the
-// volatility (1 +- 1e-6), which multiplies only the mean-zero increment: it biases no drift.
-__device__ __forceinline__ float dupire_vol(const KParams& p, float x, float t) {
+// + at}, x = S/S0 and at = -alpha t log2(e) (step number times KParams::dup_f or dup_c), with the hardware's
+// approximate base-2 logarithm and exponential (`lg2.approx.ftz.f32`, `ex2.approx.ftz.f32`: errors about
+// 2^-22, the same special values: log2 of 0 is -inf, of a negative x NaN, 2^-inf = 0).  As with the Heston
+// square root, the error scales the volatility (1 +- 1e-6), which multiplies only the mean-zero
+// increment: it biases no drift.
+__device__ __forceinline__ float dupire_vol(const KParams& p, float x, float at) {
     float l, e;
-    asm("lg2.approx.f32 %0, %1;" : "=f"(l) : "f"(x));
-    const float a = fmaf(p.bm1, l, -p.alpha * t * kLog2e);
-    asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(a));
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));
+    const float a = fmaf(p.bm1, l, at);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(a));
     return p.sigma0 * e;
 }
 
@@ -370,14 +374,14 @@ struct Leg {
         else if constexpr (PAY == PAY_LOOKBACK || PAY == PAY_DOWNOUT) r0 = on ? fminf(r0, S) : r0;
         else if constexpr (PAY == PAY_UPOUT) r0 = on ? fmaxf(r0, S) : r0;
     }
-    // t = ks h is step ks's time (the grid local-vol model reads its time row ks instead)
+    // at: step ks's time in the parametric volatility's exponent (the grid model reads its time row ks)
     template <bool RUN>
-    __device__ __forceinline__ void step(const KParams& p, float dw1, float dw2, float t,
+    __device__ __forceinline__ void step(const KParams& p, float dw1, float dw2, float at,
                                          float muh, float omk, float hstep, int ks) {
         if constexpr (MOD == MOD_GBM) {
             S = fmaf(S, fmaf(p.sigma, dw1, muh), S);
         } else if constexpr (MOD == MOD_DUPIRE) {
-            const float sl = dupire_vol(p, S * p.inv_S0, t);
+            const float sl = dupire_vol(p, S * p.inv_S0, at);
             S = fmaf(S, fmaf(sl, dw1, muh), S);
         } else if constexpr (MOD == MOD_LVGRID) {
             const float sl = lv_sigma_row(p, S, __ldg(p.lv_rows + ks));
@@ -450,7 +454,7 @@ struct PathC {
     }
     // one fine step and, coupled, its increments summed for the coarse step
     __device__ __forceinline__ void fine_dw(const KParams& p, float dw1, float dw2) {
-        const float t = (float)k * p.h;
+        const float t = (float)k * p.dup_f;
         if constexpr (HES && COUPLED) {   // run_upd is a runtime flag only here
             f.template step<false>(p, dw1, dw2, t, muh_f, p.om_f, p.h, k);
             if constexpr (path_dep<PAY>()) f.update_if(run_upd);
@@ -465,7 +469,7 @@ struct PathC {
     }
     // the coarse step on the last M fine increments
     __device__ __forceinline__ void coarse_now(const KParams& p) {
-        const float tc = (float)ck * p.hc;
+        const float tc = (float)ck * p.dup_c;
         if constexpr (HES) {
             c.template step<false>(p, a1, a2, tc, muh_c, p.om_c, p.hc, ck);
             if constexpr (path_dep<PAY>()) c.update_if(run_upd);
@@ -500,21 +504,19 @@ struct PathC {
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             const float z1 = z[2 * i], z2 = z[2 * i + 1];
-            fine_dw(p, z1 * p.sqrt_h, fmaf(p.L10, z1, p.L11 * z2) * p.sqrt_h);
+            fine_dw(p, z1 * p.sqrt_h, fmaf(p.L10s, z1, p.L11s * z2));
             if ((i % MM) == MM - 1) coarse_now(p);
         }
     }
+    // two Heston steps from a float4 of a transposed tile
     template <int MM>
     __device__ __forceinline__ void tile_smem_mm(const KParams& p, const float4* row4, int lane) {
-#pragma unroll 1
-        for (int c2 = 0; c2 < 4; c2++) {
-#pragma unroll
-            for (int cc = 0; cc < 2; cc++) {
-                const float4 v = row4[(2 * c2 + cc) ^ (lane & 7)];
-                fine_dw(p, v.x * p.sqrt_h, fmaf(p.L10, v.x, p.L11 * v.y) * p.sqrt_h);
-                fine_dw(p, v.z * p.sqrt_h, fmaf(p.L10, v.z, p.L11 * v.w) * p.sqrt_h);
-                if (MM == 2 || cc == 1) coarse_now(p);   // after fine steps 2 (M = 2) or 4 (M = 4)
-            }
+#pragma unroll 2
+        for (int c = 0; c < 8; c++) {
+            const float4 v = row4[c ^ (lane & 7)];
+            fine_dw(p, v.x * p.sqrt_h, fmaf(p.L10s, v.x, p.L11s * v.y));
+            fine_dw(p, v.z * p.sqrt_h, fmaf(p.L10s, v.z, p.L11s * v.w));
+            if (MM == 2 || (MM == 4 && (c & 1))) coarse_now(p);
         }
     }
     // raw normals, tile of 32 dimensions starting at a tile boundary
@@ -529,14 +531,14 @@ struct PathC {
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
                         const float z1 = z[2 * i], z2 = z[2 * i + 1];
-                        step_dw(p, z1 * p.sqrt_h, fmaf(p.L10, z1, p.L11 * z2) * p.sqrt_h);
+                        step_dw(p, z1 * p.sqrt_h, fmaf(p.L10s, z1, p.L11s * z2));
                     }
                 }
             } else if constexpr (HES) {
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const float z1 = z[2 * i], z2 = z[2 * i + 1];
-                    step_dw(p, z1 * p.sqrt_h, fmaf(p.L10, z1, p.L11 * z2) * p.sqrt_h);
+                    step_dw(p, z1 * p.sqrt_h, fmaf(p.L10s, z1, p.L11s * z2));
                 }
             } else if constexpr (MOD == MOD_GBM && !COUPLED) {
                 const float sig_sqh = p.sigma * p.sqrt_h;
@@ -562,7 +564,7 @@ struct PathC {
                 for (int i = 0; i < 16; i++)
                     if (2 * i < nv) {
                         const float z1 = z[2 * i], z2 = z[2 * i + 1];
-                        step_dw(p, z1 * p.sqrt_h, fmaf(p.L10, z1, p.L11 * z2) * p.sqrt_h);
+                        step_dw(p, z1 * p.sqrt_h, fmaf(p.L10s, z1, p.L11s * z2));
                     }
             } else {
 #pragma unroll
@@ -574,24 +576,24 @@ struct PathC {
     }
     // Heston: the same steps fed straight from this lane's row of a transposed tile in shared
     // memory, four normals (two steps) per float4 and the chunk loop rolled; the fully unrolled
-    // sixteen steps of tile() (fine and coarse legs) weighed on the instruction cache
+    // sixteen steps of tile() (fine and coarse legs) weighed on the instruction cache.  (GBM and Dupire
+    // keep tile(): from shared memory they were 2-3 % slower.)
     static constexpr bool SMEM_TILE = HES;
     __device__ __forceinline__ void tile_smem(const KParams& p, const float* buf, int lane, int nv) {
         const float4* row4 = reinterpret_cast<const float4*>(buf + lane * 32);
-        if constexpr (COUPLED) {
-            if (nv == 32 && m == 0 && (p.M == 2 || p.M == 4)) {
-                if (p.M == 2) tile_smem_mm<2>(p, row4, lane);
-                else tile_smem_mm<4>(p, row4, lane);
-                flush();
-                return;
-            }
+        if (nv == 32 && (!COUPLED || (m == 0 && (p.M == 2 || p.M == 4)))) {
+            if (!COUPLED) tile_smem_mm<0>(p, row4, lane);
+            else if (p.M == 2) tile_smem_mm<2>(p, row4, lane);
+            else tile_smem_mm<4>(p, row4, lane);
+            flush();
+            return;
         }
 #pragma unroll 2
         for (int c = 0; c < 8; c++) {
             if (4 * c < nv) {
                 const float4 v = row4[c ^ (lane & 7)];
-                step_dw(p, v.x * p.sqrt_h, fmaf(p.L10, v.x, p.L11 * v.y) * p.sqrt_h);
-                if (4 * c + 2 < nv) step_dw(p, v.z * p.sqrt_h, fmaf(p.L10, v.z, p.L11 * v.w) * p.sqrt_h);
+                step_dw(p, v.x * p.sqrt_h, fmaf(p.L10s, v.x, p.L11s * v.y));
+                if (4 * c + 2 < nv) step_dw(p, v.z * p.sqrt_h, fmaf(p.L10s, v.z, p.L11s * v.w));
             }
         }
         flush();
@@ -656,8 +658,7 @@ struct CvDupireC {
         Sd = Sg = p.S0; muh = p.mu * p.h; k = 0;
     }
     __device__ __forceinline__ void step_dw(const KParams& p, float dw, float) {
-        const float t = (float)k * p.h;
-        const float sl = dupire_vol(p, Sd * p.inv_S0, t);
+        const float sl = dupire_vol(p, Sd * p.inv_S0, (float)k * p.dup_f);
         Sd = fmaf(Sd, fmaf(sl, dw, muh), Sd);
         Sg = fmaf(Sg, fmaf(p.ctrl_sigma, dw, muh), Sg);
         k++;
@@ -736,7 +737,7 @@ struct BasketC {
                 if (a >= f && a < n) dw[a] = fmaf(__ldg(Lrow + a * n), x, dw[a]);
         }
         if (++f == n) {
-            const float t = (float)k * p.h;
+            const float t = (float)k * p.dup_f;
 #pragma unroll
             for (int a = 0; a < NB; a++) {
                 if (a < n) {
@@ -808,7 +809,7 @@ struct BasketTileC {
                     const float4 v = row4[(col >> 2) ^ (lane & 7)];
                     x[c] = ((col & 3) == 0 ? v.x : (col & 3) == 1 ? v.y : (col & 3) == 2 ? v.z : v.w) * p.sqrt_h;
                 }
-                const float t = (float)k * p.h;
+                const float t = (float)k * p.dup_f;
 #pragma unroll
                 for (int a = N - 1; a >= 0; a--) {   // the last asset first: x[a] is not needed after asset a
                     float dw = x[a];
@@ -921,7 +922,7 @@ struct BasketLevelC {
         }
         if (++f == n) {
             const bool coarse = (++m == p.M);
-            const float t = (float)k * p.h, tc = (float)kc * p.hc;
+            const float t = (float)k * p.dup_f, tc = (float)kc * p.dup_c;
 #pragma unroll
             for (int a = 0; a < NB; a++) {
                 if (a < n) {
@@ -1011,7 +1012,7 @@ struct BasketWideC {
             for (int a = f; a < n; a++) dw[a] = fmaf(__ldg(Lcol + a * n), x, dw[a]);
         }
         if (++f == n) {
-            const float t = (float)k * p.h;
+            const float t = (float)k * p.dup_f;
 #pragma unroll 1
             for (int a = 0; a < n; a++) {
                 if constexpr (MOD == MOD_MULTI) {
@@ -1118,7 +1119,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
             if constexpr (GEN == GEN_SOBOL) {
                 uint32_t* slot = carry ? carry + s0 + lane : nullptr;
                 if constexpr (PLAIN) sobol_tile_plain(dr, p.dstride, d0 + lane, lane < nv, h, p.u_cap, buf, lane, slot, cont);
-                else sobol_tile<PARITY>(dr, p.dstride, d0 + lane, lane < nv, h, p.u_cap, buf, lane, slot, cont);
+                else sobol_tile<PARITY>(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, slot, cont);
                 __syncwarp();
                 if constexpr (smem_tile_of<C>::value) {
                     cons.tile_smem(p, buf, lane, nv);
@@ -1139,7 +1140,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
         // N <= 32 (one tile): dW_i = sum_k M[i][k] z_k with z and M rounded to fp16 as the
         // reference's cast + GEMM (methods_cuda.cu:1228-1229); larger N runs in k_pca.
         const int N = D;
-        sobol_tile<PARITY>(dr, p.dstride, lane, lane < N, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
+        sobol_tile<PARITY>(dr, p.dstride, lane, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
         __syncwarp();
         float z[32];
         read_row(buf, lane, z);
@@ -1174,7 +1175,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
         const int N = D;
         if (N <= 32) {
             // one tile: the literal table-driven bridge (bb_apply, utils.cpp:104-124)
-            sobol_tile<PARITY>(dr, p.dstride, lane, lane < N, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
+            sobol_tile<PARITY>(dr, p.dstride, lane, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
             __syncwarp();
             float z[32];
             read_row(buf, lane, z);
@@ -1202,7 +1203,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
             // carry slots: the skeleton tiles first, then one per window
             const int ns = (S + 31) & ~31;
             for (int t0 = 0; t0 < S; t0 += 32) {
-                sobol_tile<PARITY>(dr, p.dstride, t0 + lane, t0 + lane < S, h, p.u_cap, buf, lane,
+                sobol_tile<PARITY>(dr, p.dstride, t0 + lane, h, p.u_cap, buf, lane,
                            carry ? carry + t0 + lane : nullptr, cont);
                 __syncwarp();
                 float z[32];
@@ -1222,12 +1223,11 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
             }
             for (int q = 0; q < S; q++) {
                 int dim = 0;
-                const bool act = lane < 31;
-                if (act) {
+                if (lane < 31) {   // (lane 31: dimension 0 again)
                     const int u = 31 - __clz(lane + 1);
                     dim = (S << u) + (q << u) + (lane + 1 - (1 << u));
                 }
-                sobol_tile<PARITY>(dr, p.dstride, dim, act, h, p.u_cap, buf, lane,
+                sobol_tile<PARITY>(dr, p.dstride, dim, h, p.u_cap, buf, lane,
                            carry ? carry + ns + 32 * q + lane : nullptr, cont);
                 __syncwarp();
                 float z[32];
@@ -1337,7 +1337,7 @@ __device__ __forceinline__ void assisted_pass(const KParams& p, unsigned char* s
                     }
                     float* b = ring + s * 1024;
                     if constexpr (GEN == GEN_SOBOL) {
-                        sobol_tile(dr, p.dstride, 32 * t + lane, 32 * t + lane < D, h, p.u_cap, b, lane);
+                        sobol_tile(dr, p.dstride, 32 * t + lane, h, p.u_cap, b, lane);
                     } else {
                         float z[32];
                         philox_tile(p.seed, stream, h * 32 + (uint64_t)lane, t, z);
@@ -1404,8 +1404,7 @@ __global__ void __launch_bounds__(kThreads, MINB ? MINB : (noise_is_bb(NOISE) ? 
             const int D = p.D, Q = 32 / D;
             const int qj = lane / D, dj = lane - qj * D;
             for (uint64_t h = gb; h < ge; h += (uint64_t)Q) {
-                const uint64_t hl = h + (uint64_t)qj;
-                sobol_tile(dr, p.dstride, dj, qj < Q && hl < ge, hl, p.u_cap, buf, lane);
+                sobol_tile(dr, p.dstride, dj, min(h + (uint64_t)qj, ge - 1), p.u_cap, buf, lane);
                 __syncwarp();
                 const int nq = (int)min((uint64_t)Q, ge - h);
                 for (int q = 0; q < nq; q++) {

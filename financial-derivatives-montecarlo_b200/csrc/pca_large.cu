@@ -34,7 +34,7 @@ constexpr long long kBatchFloats = 1LL << 27;   // Z: 256 MB fp16, dW: 512 MB fp
 // One warp per (32-point group, 32-dimension tile): the tile's normals through the transpose
 // buffer, then lane l writes point 32h + l of each of the 32 dimensions (consecutive rows per
 // dimension: coalesced).
-__global__ void __launch_bounds__(kThreads) k_pca_normals(const uint32_t* __restrict__ dr, int N, uint64_t g0,
+__global__ void __launch_bounds__(kThreads) k_pca_normals(const uint32_t* __restrict__ dr, int dstride, int N, uint64_t g0,
                                                          uint64_t G, uint64_t offset, uint64_t n_points,
                                                          float u_cap, __half* __restrict__ Z, int ldz) {
     __shared__ float4 smem4[(kWarpsPerBlock * kTileBytes + kTilePad) / 16];
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kThreads) k_pca_normals(const uint32_t* __rest
          t += (uint64_t)gridDim.x * kWarpsPerBlock) {
         const uint64_t h = g0 + t / (uint64_t)ntiles;
         const int d0 = (int)(t % (uint64_t)ntiles) * 32;
-        sobol_tile(dr, N, d0 + lane, d0 + lane < N, h, u_cap, buf, lane);
+        sobol_tile(dr, dstride, d0 + lane, h, u_cap, buf, lane);
         __syncwarp();
         float z[32];
         read_row(buf, lane, z);
@@ -91,7 +91,8 @@ void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* 
     cublasHandle_t blas = static_cast<cublasHandle_t>(ws.blas.h);
     cublas_check(cublasSetStream(blas, ws.stream), "set stream");
 
-    const uint32_t* dirs = direction_table(ws, a.salt0, R, N, false);
+    const int Nt = table_dims(N, 32);
+    const uint32_t* dirs = direction_table(ws, a.salt0, R, Nt, false);
     const uint64_t pb = std::max<uint64_t>(32, (uint64_t)(kBatchFloats / N) / 32 * 32);
     const uint64_t pfirst = std::min<uint64_t>(pb, (a.n_points + 31) / 32 * 32);
     __half* Z = (__half*)ws.pca_z.ensure(sizeof(__half) * (size_t)pfirst * N);
@@ -102,7 +103,7 @@ void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* 
     KernelInfo& ki = kernel_info(fn, csmem);
     const float one = 1.0f, zero = 0.0f;
     for (int r = 0; r < R; r++) {
-        const uint32_t* dr = dirs + (size_t)r * kDirRows * N;
+        const uint32_t* dr = dirs + (size_t)r * kDirRows * Nt;
         for (uint64_t o = a.offset; o < a.offset + a.n_points; o += pb) {
             const uint64_t nb = std::min<uint64_t>(pb, a.offset + a.n_points - o);
             const int ld = (int)((nb + 31) / 32 * 32);
@@ -112,7 +113,7 @@ void pca_large_pass_async(Workspace& ws, const PassArgs& a, KParams& k, double* 
             const long long gblocks = std::min<long long>((long long)((tasks + kWarpsPerBlock - 1) / kWarpsPerBlock),
                                                           (long long)E.sm_count * 8);
             k_pca_normals<<<(unsigned)std::max<long long>(gblocks, 1), kThreads, 0, ws.stream>>>(
-                dr, N, g0, G, o, nb, k.u_cap, Z, ld);
+                dr, Nt, N, g0, G, o, nb, k.u_cap, Z, ld);
             MCQ_CUDA(cudaGetLastError());
             // dW (ld x N, column-major) = Z (ld x N) * B, B(k, i) = M[i][k] = table[i * N + k]
             cublas_check(cublasGemmEx(blas, CUBLAS_OP_N, CUBLAS_OP_N, ld, N, N, &one, Z, CUDA_R_16F, ld, a.pca->table.p,
