@@ -134,7 +134,7 @@ __device__ __forceinline__ void sobol_tile_to_A(const uint32_t* __restrict__ dr,
                                                 uint64_t h, float u_cap, unsigned char* A,
                                                 int row0, int e) {
     const uint32_t base = smem_u32(A + row0 * 128) ^ (uint32_t)(((e >> 3) << 4) | ((e & 7) * 2));
-    TileWalk w = tile_walk(dr, D, dim, h, base, nullptr, 0);
+    TileWalk w = tile_walk(dr, D, dim, h, base, 0, false);
     all_strata<PARITY>(
         w, u_cap,
         [](uint32_t a, float z) {

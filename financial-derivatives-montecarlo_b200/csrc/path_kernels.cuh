@@ -107,21 +107,23 @@ __device__ __forceinline__ void read_row(const float* buf, int lane, float (&z)[
 //
 // Packed start word of group h: shift ^ W_{5+k} over the set bits k of gray(h), and, for odd h,
 // the row 31 that bit 4 of gray(32h) contributes.  A caller that generates the same dimension for groups
-// h - 1, h, h + 1, ... in order keeps the packed word of each tile in `slot` (shared memory) and passes
-// cont = 1 from the second group on: one word instead of the walk and its chain of dependent loads.
-// cont = 2: the slot already holds group h's word (a tile generated again for the same group, as the
-// adjoint's reverse sweep does).
+// h - 1, h, h + 1, ... in order keeps the packed word of each tile in the shared-memory word at address `slot` (0:
+// none) and passes cont from the second group on: one word instead of the walk and its chain of
+// dependent loads.
 struct TileWalk {
     uint32_t x, a;          // point and shared-memory address of the current stratum
     uint2 R0, R1, R2, R3, R4;   // .x: R_k, .y: the row bits of its row
 };
 
-// The packed word of group h's point of stratum 0 (slot and cont as above, without the store).
+// The packed word of group h's point of stratum 0.
 __device__ __forceinline__ uint32_t start_word(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
-                                               const uint32_t* slot, int cont) {
+                                               uint32_t slot, bool cont) {
     const uint32_t* col = dr + dim;
-    if (slot != nullptr && cont == 2) return *slot;
-    if (slot != nullptr && cont) return *slot ^ 0xF8000000u ^ __ldg(col + (kDirRowW5 - 1 + __ffsll((long long)h)) * D);
+    if (cont) {
+        uint32_t w;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(slot));
+        return w ^ 0xF8000000u ^ __ldg(col + (kDirRowW5 - 1 + __ffsll((long long)h)) * D);
+    }
     uint32_t s = __ldg(col + kDirRowShift * D) ^ (0u - ((uint32_t)h & 1u) & 0xF8000000u);
     uint32_t g = (uint32_t)(h ^ (h >> 1));
     while (g) {
@@ -132,7 +134,7 @@ __device__ __forceinline__ uint32_t start_word(const uint32_t* __restrict__ dr, 
 }
 
 __device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
-                                              uint32_t base, uint32_t* slot, int cont) {
+                                              uint32_t base, uint32_t slot, bool cont) {
     const uint2* rk = reinterpret_cast<const uint2*>(dr) + dim;
     TileWalk w;
     w.R0 = __ldg(rk);
@@ -141,7 +143,7 @@ __device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, i
     w.R3 = __ldg(rk + 3 * D);
     w.R4 = __ldg(rk + 4 * D);
     const uint32_t s = start_word(dr, D, dim, h, slot, cont);
-    if (slot != nullptr) *slot = s;
+    if (slot) asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot), "r"(s) : "memory");
     w.x = s & 0x07FFFFFFu;
     w.a = base ^ row_bits(s >> 27);
     return w;
@@ -173,8 +175,8 @@ __device__ __forceinline__ void all_strata(TileWalk& w, float u_cap, const STORE
 // instructions per normal.
 template <bool PARITY = false>
 __device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
-                                           float u_cap, float* buf, int lane, uint32_t* slot = nullptr,
-                                           int cont = 0) {
+                                           float u_cap, float* buf, int lane, uint32_t slot = 0,
+                                           bool cont = false) {
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(buf) ^ ((uint32_t)lane << 2);
     TileWalk w = tile_walk(dr, D, dim, h, base, slot, cont);
     all_strata<PARITY>(
@@ -1112,14 +1114,19 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
                                           bool cont = false) {
     const int D = p.D;
     constexpr bool PARITY = parity_of<C>::value;
+    // this lane's first slot as a shared-memory address (0: no slots)
+    const uint32_t slots = carry ? (uint32_t)__cvta_generic_to_shared(carry + lane) : 0u;
+    const bool again = slots != 0 && cont;
     if constexpr (NOISE == NOISE_RAW) {
         constexpr int TD = tile_dims_of<C>::value;   // dimensions a tile holds (32 except for baskets)
         for (int d0 = 0, s0 = 0; d0 < D; d0 += TD, s0 += 32) {
             const int nv = min(TD, D - d0);
             if constexpr (GEN == GEN_SOBOL) {
-                uint32_t* slot = carry ? carry + s0 + lane : nullptr;
-                if constexpr (PLAIN) sobol_tile_plain(dr, p.dstride, d0 + lane, lane < nv, h, p.u_cap, buf, lane, slot, cont);
-                else sobol_tile<PARITY>(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, slot, cont);
+                if constexpr (PLAIN)
+                    sobol_tile_plain(dr, p.dstride, d0 + lane, lane < nv, h, p.u_cap, buf, lane,
+                                     carry ? carry + s0 + lane : nullptr, cont);
+                else
+                    sobol_tile<PARITY>(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, slots ? slots + 4 * s0 : 0, again);
                 __syncwarp();
                 if constexpr (smem_tile_of<C>::value) {
                     cons.tile_smem(p, buf, lane, nv);
@@ -1140,7 +1147,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
         // N <= 32 (one tile): dW_i = sum_k M[i][k] z_k with z and M rounded to fp16 as the
         // reference's cast + GEMM (methods_cuda.cu:1228-1229); larger N runs in k_pca.
         const int N = D;
-        sobol_tile<PARITY>(dr, p.dstride, lane, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
+        sobol_tile<PARITY>(dr, p.dstride, lane, h, p.u_cap, buf, lane, slots, again);
         __syncwarp();
         float z[32];
         read_row(buf, lane, z);
@@ -1175,7 +1182,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
         const int N = D;
         if (N <= 32) {
             // one tile: the literal table-driven bridge (bb_apply, utils.cpp:104-124)
-            sobol_tile<PARITY>(dr, p.dstride, lane, h, p.u_cap, buf, lane, carry ? carry + lane : nullptr, cont);
+            sobol_tile<PARITY>(dr, p.dstride, lane, h, p.u_cap, buf, lane, slots, again);
             __syncwarp();
             float z[32];
             read_row(buf, lane, z);
@@ -1204,7 +1211,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
             const int ns = (S + 31) & ~31;
             for (int t0 = 0; t0 < S; t0 += 32) {
                 sobol_tile<PARITY>(dr, p.dstride, t0 + lane, h, p.u_cap, buf, lane,
-                           carry ? carry + t0 + lane : nullptr, cont);
+                           slots ? slots + 4 * t0 : 0, again);
                 __syncwarp();
                 float z[32];
                 read_row(buf, lane, z);
@@ -1228,7 +1235,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
                     dim = (S << u) + (q << u) + (lane + 1 - (1 << u));
                 }
                 sobol_tile<PARITY>(dr, p.dstride, dim, h, p.u_cap, buf, lane,
-                           carry ? carry + ns + 32 * q + lane : nullptr, cont);
+                           slots ? slots + 4 * (ns + 32 * q) : 0, again);
                 __syncwarp();
                 float z[32];
                 read_row(buf, lane, z);
