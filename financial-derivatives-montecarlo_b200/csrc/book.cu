@@ -49,7 +49,21 @@ constexpr int kMaxChunksPerRep = 1024;
 constexpr int kHdrChunk0 = 2;
 constexpr int kHdrSlice0 = kHdrChunk0 + kBookClasses + 1;
 constexpr int kHdrCounter0 = kHdrSlice0 + kBookClasses + 1;
-constexpr int kHdrInts = kHdrCounter0 + kBookClasses;
+// [kHdrStored0 + l] points of level l whose normals are stored (below).
+constexpr int kHdrStored0 = kHdrCounter0 + kBookClasses;
+constexpr int kHdrInts = kHdrStored0 + kBookMaxLevels;
+
+// Stored normals.  Every option of a level draws replica r's points from the same table, so in a batched
+// round the normals of the points that several options are about to use are formed once, written to
+// device memory and read by all of them (the same bits): generation is about 60 % of a basket path's
+// instructions.  A block holds kStoreGroups 32-point groups of all replicas and of the level's first dims
+// dimensions, [replica][dimension][1024 points]; blocks are carved from slabs of kStoreSlab bytes that the
+// engine keeps until mcq_shutdown (at most kStoreMaxBytes, and an eighth of the free device memory; a book
+// takes only what it fills).  48 baskets at eps 2.5e-3, two books: 247 and 174 ms without a store, 220 and 148 with
+// 8 GiB, 204 and 134 with 16, 191-205 and 128-138 with 24.
+constexpr int kStoreGroups = 32, kStorePoints = 32 * kStoreGroups;
+constexpr int kStoreMaxBlocks = 1 << 14;   // per level
+constexpr size_t kStoreSlab = (size_t)1 << 30, kStoreMaxBytes = (size_t)16 << 30;
 
 struct BookOptDev {
     double T;
@@ -74,6 +88,8 @@ struct BookArgs {
     int dstride[kBookMaxLevels];
     int R, M, n0;
     float u_cap;
+    const float* const* stored;     // [level][kStoreMaxBlocks] blocks of stored normals
+    int stored_dims[kBookMaxLevels];
     double* records;      // [chunk][kBookNST]
     double* out;          // [slice][kBookOut]
 };
@@ -285,7 +301,36 @@ __device__ __forceinline__ void book_chunk(const BookArgs& a, const BookSpec& s,
     const uint64_t pend = (uint64_t)s.offset + s.n_points;
     const float4* L4 = reinterpret_cast<const float4*>(Ls);
     __syncwarp();
-    if (D <= 8 && 2 * Dt <= 32) {   // wider baskets keep their registers for the step-major path
+    if (ge * 32 <= (uint64_t)a.hdr[kHdrStored0 + s.level]) {
+        // stored normals: one coalesced load per normal, the next step's on their way during this one
+        const float* const* blocks = a.stored + (size_t)s.level * kStoreMaxBlocks;
+        const size_t rep = (size_t)r * (size_t)a.stored_dims[s.level] * kStorePoints + (size_t)lane;
+        auto group_base = [&](uint64_t g) { return blocks[g / kStoreGroups] + rep + (g % kStoreGroups) * 32; };
+        const float* z = group_base(gb);
+        float x[D];
+#pragma unroll
+        for (int c = 0; c < D; c++) x[c] = __ldcs(z + c * kStorePoints);
+        for (uint64_t g = gb; g < ge; g++) {
+            P path;
+            path.init(sg);
+            for (int k = 0; k < nf; k++) {
+                const bool last = k + 1 == nf;
+                if (last && g + 1 < ge) z = group_base(g + 1);
+                const float* zn = z + (last ? 0 : (size_t)(k + 1) * D * kStorePoints);
+                float xs[D];
+#pragma unroll
+                for (int c = 0; c < D; c++) {
+                    xs[c] = x[c] * sqrt_h;
+                    x[c] = __ldcs(zn + c * kStorePoints);   // (after the chunk's last step: any stored word)
+                }
+                path.step(xs, L4, sg, muh_f, muh_c, Mc);
+            }
+            float y[NS];
+            path.finish(sg, K, disc, has_c, y);
+            const uint64_t n = g * 32 + (uint64_t)lane;
+            acc.add(y, n >= s.offset && n < pend, lane);
+        }
+    } else if (D <= 8 && 2 * Dt <= 32) {   // wider baskets keep their registers for the step-major path
         const int Q = 32 / Dt, qj = lane / Dt, dj = lane - qj * Dt;
         for (uint64_t g = gb; g < ge; g += Q) {
             const uint64_t gl = g + (uint64_t)qj;
@@ -381,6 +426,40 @@ __device__ __forceinline__ void book_chunk(const BookArgs& a, const BookSpec& s,
         }
     }
     acc.flush(rec, lane);
+}
+
+// The normals of blocks [b0, b1) of one level: a warp takes 32 dimensions of a replica for four groups, one
+// after the other through its transpose tile, and writes each dimension's 32 points as one line.
+constexpr int kStoreRun = 4;
+__global__ void __launch_bounds__(kThreads) k_book_store(const uint32_t* __restrict__ dirs, int dstride, int R, int dims,
+                                                        int b0, int b1, float u_cap, float* const* blocks) {
+    __shared__ float tile[kWarpsPerBlock][1024];
+    __shared__ uint32_t slot[kWarpsPerBlock][32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    float* buf = tile[wib];
+    const int nt = (dims + 31) >> 5;
+    const long long tasks = (long long)(b1 - b0) * R * nt * (kStoreGroups / kStoreRun);
+    for (long long t = (long long)blockIdx.x * kWarpsPerBlock + wib; t < tasks; t += (long long)gridDim.x * kWarpsPerBlock) {
+        const int d0 = (int)(t % nt) * 32, r = (int)(t / nt % R);
+        const int q = (int)(t / nt / R % (kStoreGroups / kStoreRun)), b = b0 + (int)(t / nt / R / (kStoreGroups / kStoreRun));
+        const uint32_t* dr = dirs + (size_t)r * kPlainRows * (size_t)dstride;
+        float* to = blocks[b] + ((size_t)r * dims + d0) * kStorePoints + lane;
+        const int nv = min(32, dims - d0);
+        for (int g = q * kStoreRun; g < (q + 1) * kStoreRun; g++) {
+            sobol_tile_plain(dr, dstride, d0 + lane, lane < nv, (uint64_t)b * kStoreGroups + g, u_cap, buf, lane,
+                             &slot[wib][lane], g > q * kStoreRun);
+            __syncwarp();
+#pragma unroll
+            for (int c4 = 0; c4 < 8; c4++) {
+                const float4 v = reinterpret_cast<const float4*>(buf + lane * 32)[c4 ^ (lane & 7)];
+                const float z[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (4 * c4 + c < nv) to[(size_t)(4 * c4 + c) * kStorePoints + 32 * g] = z[c];
+            }
+            __syncwarp();
+        }
+    }
 }
 
 // Persistent work-queue kernel of one width class: warps take chunks from the class's atomic
@@ -671,6 +750,12 @@ struct BookRunner {
     std::vector<DevBuf*> dirs;    // level l's table in workspace 1 + l
     std::vector<int> dstride;
     std::vector<OptState> st;
+    int stored_pts[kBookMaxLevels] = {};    // points of each level whose normals are stored
+    int basket_dmax = 0;                    // widest basket
+    std::vector<float*> h_stored;           // host copy of the block table
+    DevBuf* d_stored = nullptr;
+    size_t slab = 0, slab_at = 0;           // next free byte of the slabs
+    bool store_full = false;
     size_t max_specs = 0;
     long long launches = 0, rounds = 0;
     double path_steps = 0, normals = 0;
@@ -695,9 +780,78 @@ struct BookRunner {
         }
         a.R = R; a.M = M; a.n0 = n0;
         a.u_cap = ((qc.flags | ml.flags) & MCQ_FLAG_COMPAT_U_INF) ? 1.0f : 0x1.fffffep-1f;
+        a.stored = d_stored ? (const float* const*)d_stored->p : nullptr;
+        for (int l = 0; l <= max_L_all; l++) a.stored_dims[l] = (int)(basket_dmax * nfine(l));
         a.records = (double*)s.records.p;
         a.out = (double*)s.out.p;
         return a;
+    }
+
+    // Room for one block in the engine's slabs; nullptr when the store is full.
+    float* store_block(size_t bytes) {
+        auto& slabs = engine().store_slabs;
+        if (store_full || bytes > kStoreSlab) return nullptr;
+        if (slab_at + bytes > kStoreSlab) { slab++; slab_at = 0; }
+        if (slab >= slabs.size()) {
+            store_full = true;   // unless another slab is to be had
+            if ((slab + 1) * kStoreSlab > kStoreMaxBytes) return nullptr;
+            size_t free_b = 0, total = 0;
+            MCQ_CUDA(cudaMemGetInfo(&free_b, &total));
+            if ((slab + 1) * kStoreSlab > (free_b + slabs.size() * kStoreSlab) / 8) return nullptr;
+            auto b = std::make_unique<DevBuf>();
+            try { b->ensure(kStoreSlab); } catch (const Error&) { return nullptr; }
+            slabs.push_back(std::move(b));
+            store_full = false;
+        }
+        float* p = (float*)((char*)slabs[slab]->p + slab_at);
+        slab_at += bytes;
+        return p;
+    }
+
+    // Before a round: store the normals of each level up to the point that a sixth of its slices (at least
+    // three) still reach, where the slices draw at least four times the normals that this adds.  (A normal
+    // stored costs its generation once and 4 bytes written; one read saves the generation, so two would pay;
+    // from two to four the measured times are the same, and the memory goes further.)
+    void store_normals(Slot& s, const std::vector<BookSpec>& sp) {
+        for (int l = 0; l <= max_L_all; l++) {
+            std::vector<long long> ends;
+            for (const BookSpec& x : sp)
+                if (x.level == l && !opts[x.opt].model) ends.push_back((long long)x.offset + x.n_points);
+            const size_t k = std::max<size_t>(3, ends.size() / 6);
+            if (ends.size() < k) continue;
+            std::nth_element(ends.begin(), ends.begin() + (k - 1), ends.end(), std::greater<long long>());
+            const int b0 = stored_pts[l] / kStorePoints;
+            int b1 = (int)std::min<long long>((ends[k - 1] + kStorePoints - 1) / kStorePoints, kStoreMaxBlocks);
+            if (b1 <= b0) continue;
+            const long long dims = basket_dmax * nfine(l), upto = (long long)b1 * kStorePoints;
+            double drawn = 0.0;
+            for (const BookSpec& x : sp)
+                if (x.level == l && !opts[x.opt].model) {
+                    const long long a = std::max<long long>(x.offset, stored_pts[l]), e = std::min<long long>(upto, (long long)x.offset + x.n_points);
+                    if (e > a) drawn += (double)(e - a) * (double)(book_width(opts[x.opt]) * nfine(l));
+                }
+            if (drawn < 4.0 * (double)(upto - stored_pts[l]) * (double)dims) continue;
+            if (!d_stored) {
+                d_stored = &engine().ws(1).xbuf[5];
+                grow(*d_stored, sizeof(float*) * (size_t)(kBookMaxLevels * kStoreMaxBlocks));
+                h_stored.assign((size_t)kBookMaxLevels * kStoreMaxBlocks, nullptr);
+            }
+            const size_t bytes = sizeof(float) * (size_t)R * (size_t)dims * kStorePoints;
+            float** tab = h_stored.data() + (size_t)l * kStoreMaxBlocks;
+            int b = b0;
+            for (; b < b1; b++)
+                if ((tab[b] = store_block(bytes)) == nullptr) break;
+            if (b == b0) continue;
+            float** d_tab = (float**)d_stored->p + (size_t)l * kStoreMaxBlocks;
+            MCQ_CUDA(cudaMemcpyAsync(d_tab + b0, tab + b0, sizeof(float*) * (size_t)(b - b0), cudaMemcpyHostToDevice, s.stream));
+            const long long tasks = (long long)(b - b0) * R * ((dims + 31) / 32) * (kStoreGroups / kStoreRun);
+            const int grid = (int)std::min<long long>((tasks + kWarpsPerBlock - 1) / kWarpsPerBlock, (long long)engine().sm_count * 5);
+            const float cap = ((qc.flags | ml.flags) & MCQ_FLAG_COMPAT_U_INF) ? 1.0f : 0x1.fffffep-1f;
+            k_book_store<<<grid, kThreads, 0, s.stream>>>((const uint32_t*)dirs[l]->p, dstride[l], R, (int)dims, b0, b, cap, d_tab);
+            MCQ_CUDA(cudaGetLastError());
+            engine().launches++;   // (the book's own count is of its rounds' kernels)
+            stored_pts[l] = b * kStorePoints;
+        }
     }
 
     void setup() {
@@ -740,6 +894,7 @@ struct BookRunner {
                 for (int b = 0; b < d; b++) bd.push_back(o.L ? (float)o.L[a * d + b] : (a == b ? 1.f : 0.f));
             max_L_all = std::max(max_L_all, o.max_L);
             dmax = std::max(dmax, d);
+            basket_dmax = std::max(basket_dmax, d);
         }
         cudaStream_t s0 = E.ws(0).stream;
         d_opts = &E.ws(0).xbuf[5];
@@ -902,6 +1057,7 @@ struct BookRunner {
                 hs[k] = sp[k];
             }
         }
+        for (int l = 0; l < kBookMaxLevels; l++) h[kHdrStored0 + l] = stored_pts[l];
         h[0] = (int)sp.size();
         h[1] = h[kHdrChunk0 + kBookClasses] = chunk;
         h[kHdrSlice0 + kBookClasses] = (int)sp.size();
@@ -976,8 +1132,10 @@ struct BookRunner {
                 long long chunks = 0;
                 for (auto& x : sp) chunks += (long long)R * x.cpr;
                 grow(s.records, sizeof(double) * kBookNST * (size_t)std::max<long long>(chunks, 1));
+                const bool had_store = d_stored != nullptr;
+                store_normals(s, sp);
                 upload(s, sp);
-                bool var_changed = false;
+                bool var_changed = had_store != (d_stored != nullptr);
                 for (int c = 0; c < kBookClasses; c++) var_changed |= exec && var[c] != book_variant(c);
                 // (re)capture when a buffer moved or the tuner settled a class on another variant
                 if (!exec || captured_records != s.records.p || var_changed) {

@@ -112,6 +112,7 @@ void shutdown_engine() {
     if (!E.ready) return;
     cudaDeviceSynchronize();
     E.pool.clear();
+    E.store_slabs.clear();
     E.kinfo.clear();
     for (auto& kv : E.tune)
         for (auto& pr : kv.second.ev)

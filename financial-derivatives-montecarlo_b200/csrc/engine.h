@@ -125,6 +125,7 @@ struct Engine {
     std::map<std::pair<const void*, size_t>, KernelInfo> kinfo;   // occupancy per (kernel, smem)
     std::unordered_set<const void*> kattr;           // kernels whose smem limit is raised
     std::unordered_map<uint64_t, TuneState> tune;
+    std::vector<std::unique_ptr<DevBuf>> store_slabs;   // the book's stored normals (book.cu)
     int launches = 0;                                // kernel launches issued (accounting)
     int last_gpi = 0, last_carry = 0;                // work layout of the last fused pass
     Workspace& ws(int i);

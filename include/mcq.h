@@ -201,7 +201,7 @@ typedef struct mcq_book_stats {
     double  path_steps;           /* sum over slices of R x points x (fine + coarse steps) */
     double  normals;              /* sum over slices of R x points x fine steps x assets */
     int32_t rounds;               /* adaptive rounds (batched) / per-option steps (plain) */
-    int32_t launches;             /* kernel launches issued */
+    int32_t launches;             /* kernel launches of the rounds */
 } mcq_book_stats;
 
 #define MCQ_BOOK_BATCHED  0       /* every option and level in one graph replay per round */
@@ -284,7 +284,9 @@ int mcq_adjoint(const mcq_model* m, const mcq_payoff* p, int n_steps, uint32_t s
  * each option's own).  MCQ_BOOK_BATCHED runs every option's pending slices of a round in one
  * persistent work-queue kernel replayed from a CUDA graph; MCQ_BOOK_PLAIN is the per-option,
  * stream-per-level form (methods_cuda.cu:1745-1755) with the same kernels.  Both give
- * bit-identical results.  No counterpart in the reference (which rejects basket MLQMC,
+ * bit-identical results.  A batched book whose options share points keeps their normals in device
+ * memory (as much as it fills, at most 16 GiB and an eighth of what is free; given back by
+ * mcq_shutdown).  No counterpart in the reference (which rejects basket MLQMC,
  * methods_cuda.cu:1695-1697).  stats may be NULL. */
 int mcq_book_price(const mcq_book_option* opts, int n, const mcq_mlmc_cfg* ml, const mcq_qmc_cfg* qc,
                    int mode, mcq_book_result* out, mcq_book_stats* stats);
