@@ -204,6 +204,7 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
     k.sqrt_h = sqrtf(h);
     k.S0 = (float)m.S0;
     k.inv_S0 = 1.0f / k.S0;
+    k.sig_sqh = (float)(m.sigma * std::sqrt(m.T / a.n_steps));
     k.mu = (float)m.mu;
     k.sigma = (float)m.sigma;
     k.kappa = (float)m.kappa;
@@ -238,6 +239,9 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
     }
 
     k.K = (float)p.K;
+    const bool scales = m.kind == MCQ_MODEL_GBM || m.kind == MCQ_MODEL_HESTON || m.kind == MCQ_MODEL_DUPIRE;
+    const double dS = scales ? m.S0 / (double)k.S0 - 1.0 : 0.0, dK = (p.K - (double)k.K) - p.K * dS;
+    k.dK = std::isfinite(dK) && std::fabs(dK) < 1e-6 * std::fabs(p.K) ? (float)dK : 0.f;
     k.B = (float)p.B;
     k.pay_T = (float)p.T;
     switch (p.kind) {
@@ -252,6 +256,9 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
         const float sb = (float)p.sigma;
         k.corr_f = (float)std::exp((double)(-0.5826f * sb * sqrtf(h)));
         k.corr_c = (float)std::exp((double)(-0.5826f * sb * sqrtf(k.hc > 0 ? k.hc : h)));
+        const double bgk = -(double)0.5826f * p.sigma, hf = m.T / a.n_steps;
+        k.dcorr_f = (float)(std::exp(bgk * std::sqrt(hf)) - (double)k.corr_f);
+        k.dcorr_c = (float)(std::exp(bgk * std::sqrt(k.n_coarse > 0 ? m.T / k.n_coarse : hf)) - (double)k.corr_c);
     } else {
         k.corr_f = k.corr_c = 1.0f;
     }

@@ -81,6 +81,7 @@ struct KParams {
     uint64_t G;         // groups per replica
     // ---- model (single precision, as the reference's c_p)
     float S0, inv_S0, mu, T, h, sqrt_h, sigma;
+    float sig_sqh;                                 // GBM: sigma sqrt(h), rounded once
     float kappa, theta, xi, L10, L11, v0, om_f;    // om_f = 1 - exp(-kappa h), from expm1
     float L10s, L11s;                              // L10, L11 times sqrt(h)
     float sigma0, alpha, bm1;                      // Dupire: bm1 = beta_d - 1
@@ -89,6 +90,8 @@ struct KParams {
     float mil;                                     // Heston Milstein: xi^2/4 (0: Euler)
     // ---- payoff
     float K, B, disc, corr_f, corr_c, u_cap;
+    float dK;                                      // K - (float)K, less K (S0 / (float)S0 - 1) where paths scale with S0
+    float dcorr_f, dcorr_c;                        // what rounding the two corrections left out
     float pay_T;                                   // payoff maturity (discount sensitivity)
     // ---- control variate / importance sampling
     float beta_cv, E_ctrl, z_star;
