@@ -38,6 +38,12 @@ constexpr int kPcaThreads = (kPcaIssuerWarp + 1) * 32;
 constexpr int kPcaRows = 128;                // paths per tile: one M = 128 MMA
 constexpr int kPcaStages = 4;                // ring of K-block stages
 constexpr int kAStageBytes = kPcaRows * 128; // 128 rows x 64 fp16
+constexpr int kPcaCtl = 256;                 // barriers, TMEM address, failure word
+// K-blocks go round the three groups and a tile has 1, 2 or 4 of them, so a generator warp makes the same
+// dimensions of every third tile: 12 groups of 32 points on.  It keeps the packed start words of its
+// last three (one per K-block) in shared memory and XORs the few words by which gray(h - 12) and gray(h)
+// differ (2 to 4 mostly) instead of walking gray(h)'s.
+constexpr uint64_t kPcaCarry = 4 * kPcaGroups;
 constexpr uint32_t kWaitLimit = 1u << 26;    // polls of an mbarrier before giving up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
@@ -132,9 +138,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 template <bool PARITY>
 __device__ __forceinline__ void sobol_tile_to_A(const uint32_t* __restrict__ dr, int D, int dim,
                                                 uint64_t h, float u_cap, unsigned char* A,
-                                                int row0, int e) {
+                                                int row0, int e, uint32_t slot, bool cont) {
     const uint32_t base = smem_u32(A + row0 * 128) ^ (uint32_t)(((e >> 3) << 4) | ((e & 7) * 2));
-    TileWalk w = tile_walk(dr, D, dim, h, base, 0, false);
+    TileWalk w = tile_walk(dr, D, dim, base, [&] {
+        uint32_t s;
+        if (cont) {
+            const uint64_t b = h - kPcaCarry;
+            uint32_t g = (uint32_t)((h ^ (h >> 1)) ^ (b ^ (b >> 1)));
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(s) : "r"(slot));
+            while (g) {
+                s ^= __ldg(dr + dim + (kDirRowW5 - 1 + __ffs(g)) * D);
+                g &= g - 1;
+            }
+        } else {
+            s = start_word(dr, D, dim, h, 0, false);
+        }
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot), "r"(s) : "memory");
+        return s;
+    });
     all_strata<PARITY>(
         w, u_cap,
         [](uint32_t a, float z) {
@@ -159,6 +180,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
     uint64_t* done = accempty + 2;             // every MMA issued has completed
     uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tslot + 1);
+    uint32_t* starts = reinterpret_cast<uint32_t*>(sA + kPcaStages * kAStageBytes + kPcaCtl);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t ncols = (uint32_t)(2 * N);   // two accumulators of N fp32 columns
 
@@ -197,17 +219,18 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
     grid_dependency_wait();   // the factor is the handle's; the direction words are the kernel before's
     const uint32_t tbase = *tslot;
 
-    // Every role walks the same sequence: items blockIdx.x, + gridDim.x, ...; tiles [t_beg, t_end)
-    // of each item; q counts the CTA's tiles, K-block kb of tile q is the CTA's K-block q nkb + kb.
+    // Every role walks the same sequence: items [first, last), consecutive so that most tiles follow on the tile
+    // before (kPcaCarry); tiles [t_beg, t_end) of each item; q counts the CTA's tiles, K-block kb of tile q is the CTA's K-block q nkb + kb.
     const int tiles_per_rep = (int)((p.G + 3) >> 2);
-    const int n_items = p.n_items;
+    const int first = (int)((long long)p.n_items * blockIdx.x / gridDim.x);
+    const int last = (int)((long long)p.n_items * (blockIdx.x + 1) / gridDim.x);
     if (warp < kPcaDrainWarps) {
         // ---- drain warps: every tile, tile q from accumulator q mod 2
         const int quarter = warp;
         const uint32_t tlane = tbase + ((uint32_t)(32 * quarter) << 16);
         int q = 0;
         bool stop = false;
-        for (int item = blockIdx.x; item < n_items && !stop; item += gridDim.x) {
+        for (int item = first; item < last && !stop; item++) {
             const int r = item / p.items_per_rep;
             const int j = item - r * p.items_per_rep;
             const int t_beg = j * p.gpi;
@@ -246,13 +269,15 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
         //      32 rg + 31, dimensions 32 hf .. 32 hf + 31 of the K-block
         const int gi = warp - kPcaDrainWarps;
         const int rg = gi & 3, hf = (gi >> 2) & 1, grp = gi >> 3;
-        int q = 0;
+        const uint32_t slots = smem_u32(starts) + (uint32_t)(gi * nkb * 32 + lane) * 4;
+        int q = 0, q_rep = 0, rep = -1;   // q_rep: the CTA's first tile of replica rep
         bool stop = false;
-        for (int item = blockIdx.x; item < n_items && !stop; item += gridDim.x) {
+        for (int item = first; item < last && !stop; item++) {
             const int r = item / p.items_per_rep;
             const int j = item - r * p.items_per_rep;
             const int t_beg = j * p.gpi;
             const int t_end = min(t_beg + p.gpi, tiles_per_rep);
+            if (r != rep) { rep = r; q_rep = q; }
             const uint32_t* dr = p.dirs + (size_t)r * kDirRows * (size_t)N;
             for (int t = t_beg; t < t_end && !stop; t++, q++) {
                 const uint64_t h = p.g0 + (uint64_t)t * 4 + (uint64_t)rg;
@@ -265,7 +290,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
                         if (!__all_sync(0xffffffffu, ok && !*s_fail)) { *s_fail = 1; stop = true; break; }
                     }
                     sobol_tile_to_A<parity_of<C>::value>(dr, N, kb * 64 + 32 * hf + lane, h, p.u_cap, sA + s * kAStageBytes, 32 * rg,
-                                    32 * hf + lane);
+                                    32 * hf + lane, slots + kb * 128, q - q_rep >= kPcaGroups);
                     fence_proxy_async();   // generic-proxy stores visible to the tensor core's reads
                     mbar_arrive(smem_u32(&full[s]));
                 }
@@ -277,7 +302,7 @@ __global__ void __launch_bounds__(kPcaThreads, 1) k_pca(const __grid_constant__ 
         const uint32_t sB_addr = smem_u32(sB), sA_addr = smem_u32(sA);
         int q = 0;
         bool stop = false;
-        for (int item = blockIdx.x; item < n_items && !stop; item += gridDim.x) {
+        for (int item = first; item < last && !stop; item++) {
             const int j = item - (item / p.items_per_rep) * p.items_per_rep;
             const int t_beg = j * p.gpi;
             const int t_end = min(t_beg + p.gpi, tiles_per_rep);
@@ -356,7 +381,7 @@ const void* lookup_pca(int model, int payoff, bool coupled) {
     }
 }
 
-size_t pca_smem_bytes(int N) { return (size_t)N * N * 2 + (size_t)kPcaStages * kAStageBytes + 256 + kTilePad; }
+size_t pca_smem_bytes(int N) { return (size_t)N * N * 2 + (size_t)kPcaStages * kAStageBytes + kPcaCtl + (size_t)kPcaGenWarps * (N >> 6) * 128 + kTilePad; }
 int pca_threads() { return kPcaThreads; }
 int pca_warps() { return kPcaDrainWarps; }
 int pca_tile_paths() { return kPcaRows; }

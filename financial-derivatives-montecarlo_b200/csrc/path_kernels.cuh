@@ -133,8 +133,10 @@ __device__ __forceinline__ uint32_t start_word(const uint32_t* __restrict__ dr, 
     return s;
 }
 
-__device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h,
-                                              uint32_t base, uint32_t slot, bool cont) {
+// The walk from packed word START() of the tile at `base`.
+template <class START>
+__device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, int D, int dim, uint32_t base,
+                                              const START& start) {
     const uint2* rk = reinterpret_cast<const uint2*>(dr) + dim;
     TileWalk w;
     w.R0 = __ldg(rk);
@@ -142,8 +144,7 @@ __device__ __forceinline__ TileWalk tile_walk(const uint32_t* __restrict__ dr, i
     w.R2 = __ldg(rk + 2 * D);
     w.R3 = __ldg(rk + 3 * D);
     w.R4 = __ldg(rk + 4 * D);
-    const uint32_t s = start_word(dr, D, dim, h, slot, cont);
-    if (slot) asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot), "r"(s) : "memory");
+    const uint32_t s = start();
     w.x = s & 0x07FFFFFFu;
     w.a = base ^ row_bits(s >> 27);
     return w;
@@ -178,7 +179,11 @@ __device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int 
                                            float u_cap, float* buf, int lane, uint32_t slot = 0,
                                            bool cont = false) {
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(buf) ^ ((uint32_t)lane << 2);
-    TileWalk w = tile_walk(dr, D, dim, h, base, slot, cont);
+    TileWalk w = tile_walk(dr, D, dim, base, [&] {
+        const uint32_t s = start_word(dr, D, dim, h, slot, cont);
+        if (slot) asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot), "r"(s) : "memory");
+        return s;
+    });
     all_strata<PARITY>(
         w, u_cap,
         [](uint32_t a, float z) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(z) : "memory"); },
