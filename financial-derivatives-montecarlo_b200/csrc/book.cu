@@ -58,7 +58,7 @@ constexpr int kHdrInts = kHdrStored0 + kBookMaxLevels;
 // device memory and read by all of them (the same bits): generation is about 60 % of a basket path's
 // instructions.  A block holds kStoreGroups 32-point groups of all replicas and of the level's first dims
 // dimensions, [replica][dimension][1024 points]; blocks are carved from slabs of kStoreSlab bytes that the
-// engine keeps until mcq_shutdown (at most kStoreMaxBytes, and an eighth of the free device memory; a book
+// engine keeps until mcq_shutdown or until another call runs out of memory (at most kStoreMaxBytes, and an eighth of the free device memory; a book
 // takes only what it fills).  48 baskets at eps 2.5e-3, two books: 247 and 174 ms without a store, 220 and 148 with
 // 8 GiB, 204 and 134 with 16, 191-205 and 128-138 with 24.
 constexpr int kStoreGroups = 32, kStorePoints = 32 * kStoreGroups;
@@ -1110,6 +1110,11 @@ struct BookRunner {
     void run_batched() {
         Engine& E = engine();
         Slot s(E.ws(0));
+        struct Busy {
+            Engine& e;
+            ~Busy() { e.store_busy = false; }
+        } busy{E};
+        E.store_busy = true;
         constexpr int kSide = kBookClasses - 1;   // class 0 runs on the main stream
         cudaStream_t side[kSide];
         cudaEvent_t fork = nullptr, join[kSide] = {};

@@ -24,6 +24,12 @@ void* DevBuf::ensure(size_t bytes) {
     release();
     size_t want = std::max<size_t>(bytes, 256);
     cudaError_t e = cudaMalloc(&p, want);
+    Engine& E = engine();
+    if (e == cudaErrorMemoryAllocation && !E.store_busy && !E.store_slabs.empty()) {
+        cudaGetLastError();   // an earlier book's normals give way to the call that needs the memory
+        E.store_slabs.clear();
+        e = cudaMalloc(&p, want);
+    }
     if (e != cudaSuccess) {
         p = nullptr;
         cudaGetLastError();
@@ -366,8 +372,7 @@ KernelInfo& kernel_info(const void* fn, size_t smem, int threads) {
 }
 
 // The autotuner.  A family of kernels compiled with nvar launch variants that differ only in
-// register allocation, scheduling or work granularity inside a launch (never in arithmetic, so
-// every variant gives the same bits) is tuned once per process: its first launches of at least
+// register allocation (never in arithmetic, so every variant gives the same bits) is tuned once per process: its first launches of at least
 // min_units work units run one variant each, timed with events on the launching stream (the
 // caller records them around its launch when *trial is set), and the variant with the least time
 // per unit is kept.  MCQ_TUNE=<v> forces variant v.

@@ -126,6 +126,7 @@ struct Engine {
     std::unordered_set<const void*> kattr;           // kernels whose smem limit is raised
     std::unordered_map<uint64_t, TuneState> tune;
     std::vector<std::unique_ptr<DevBuf>> store_slabs;   // the book's stored normals (book.cu)
+    bool store_busy = false;                            // a batched book is running on them
     int launches = 0;                                // kernel launches issued (accounting)
     int last_gpi = 0, last_carry = 0;                // work layout of the last fused pass
     Workspace& ws(int i);
