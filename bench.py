@@ -45,9 +45,9 @@ METRIC = "path-steps/s"
 # methods_cuda.cu:273), the Kahan-compensated running sum of the Asian average (4 flops).
 FLOPS_PER_PATH_STEP = 2 + 7 + 4
 SFU_PER_PATH_STEP = 1
-# The same path-step with the inverse normal counted as the AS241 central rational it evaluates
-# (7 + 7 FMA + 1 division: 29 flops): an issue model, not the algorithmic count.
-ISSUE_MODEL_FLOPS_PER_PATH_STEP = 2 + 29 + 4 + 4
+# The same path-step with the inverse normal counted as the polynomial it evaluates: degree 5 on average over
+# the strata (11 flops), u 2, Euler step 4, compensated sum 4.
+ISSUE_MODEL_FLOPS_PER_PATH_STEP = 2 + 11 + 4 + 4
 
 
 def load_engine():
@@ -714,13 +714,14 @@ def main():
                      "issue_model": {"flops_per_path_step": ISSUE_MODEL_FLOPS_PER_PATH_STEP,
                                      "achieved": achieved * ISSUE_MODEL_FLOPS_PER_PATH_STEP / FLOPS_PER_PATH_STEP,
                                      "frac": achieved * ISSUE_MODEL_FLOPS_PER_PATH_STEP / FLOPS_PER_PATH_STEP / peak_fp32,
-                                     "what": "the inverse normal counted as the 29-flop AS241 rational"},
+                                     "what": "the inverse normal counted as the 11 flops of its polynomial"},
                      "issue_active_ncu": issue,
-                     "instructions_per_path_step_ncu": 37.7,
-                     "note": "instruction-issue bound: the algorithmic count is 13 FP32 flops and one inverse "
-                             "normal per path-step, the kernel issues about 38 thread instructions per path-step "
-                             "(about 24 in CUDA's normcdfinvf, 3 in the GBM step and Asian sum, 10 in the Sobol "
-                             "generation and transpose) at the issue activity of the committed ncu capture"},
+                     "instructions_per_path_step_ncu": 18.3,
+                     "note": "bound by the shared-memory pipe and instruction issue: the algorithmic count is 13 "
+                             "FP32 flops and one inverse normal per path-step, the kernel issues about 18 thread "
+                             "instructions per path-step (a polynomial per stratum for the inverse normal, the "
+                             "Sobol walk, the transpose, 3 in the GBM step and Asian sum) at the issue activity of "
+                             "the committed ncu capture"},
         "gpu_launches": 2 * args.steps,
         "clocks": clocks,
     }

@@ -372,10 +372,10 @@ KernelInfo& kernel_info(const void* fn, size_t smem, int threads) {
 }
 
 // The autotuner.  A family of kernels compiled with nvar launch variants that differ only in
-// register allocation (never in arithmetic, so every variant gives the same bits) is tuned once per process: its first launches of at least
-// min_units work units run one variant each, timed with events on the launching stream (the
-// caller records them around its launch when *trial is set), and the variant with the least time
-// per unit is kept.  MCQ_TUNE=<v> forces variant v.
+// register allocation (never in arithmetic, so every variant gives the same bits) is tuned once per
+// process: its first launches of at least min_units work units run one variant each, timed with events on
+// the launching stream (the caller records them around its launch when *trial is set), and the variant with
+// the least time per unit is kept.  MCQ_TUNE=<v> forces variant v.
 int tune_pick(uint64_t key, int nvar, double units, double min_units, TuneState** trial) {
     Engine& E = engine();
     *trial = nullptr;
