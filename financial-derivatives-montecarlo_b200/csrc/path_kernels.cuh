@@ -190,6 +190,25 @@ __device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int 
         std::make_integer_sequence<int, 32>{});
 }
 
+// The same with the slot as a pointer, for baskets whose steps do not fill a tile: there the address form's
+// volatile accesses cost
+// more than they save (5 assets x 52 steps x 16 x 2^16 paths: 346 us a call, 307 with this one).
+__device__ __forceinline__ void sobol_tile_slot(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h, float u_cap,
+                                                float* buf, int lane, uint32_t* slot, bool cont) {
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(buf) ^ ((uint32_t)lane << 2);
+    TileWalk w = tile_walk(dr, D, dim, base, [&] {
+        const uint32_t s = slot != nullptr && cont
+                               ? *slot ^ 0xF8000000u ^ __ldg(dr + dim + (kDirRowW5 - 1 + __ffsll((long long)h)) * D)
+                               : start_word(dr, D, dim, h, 0, false);
+        if (slot != nullptr) *slot = s;
+        return s;
+    });
+    all_strata<false>(
+        w, u_cap,
+        [](uint32_t a, float z) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(z) : "memory"); },
+        std::make_integer_sequence<int, 32>{});
+}
+
 // The generator's plain form, for the estimators whose outputs turn on single paths (the book's digital
 // deltas, the adjoint's node vegas): points in order and every normal from normcdfinvf, from the plain
 // table of 33 rows (words 0..31, shift).  Lane j's start word x(32h) = shift ^ XOR of v_k over the set
@@ -1172,6 +1191,8 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
                 if constexpr (PLAIN)
                     sobol_tile_plain(dr, p.dstride, d0 + lane, lane < nv, h, p.u_cap, buf, lane,
                                      carry ? carry + s0 + lane : nullptr, cont);
+                else if constexpr (TD != 32)
+                    sobol_tile_slot(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, carry ? carry + s0 + lane : nullptr, cont);
                 else
                     sobol_tile<PARITY>(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, slots ? slots + 4 * s0 : 0, again);
                 __syncwarp();
