@@ -248,6 +248,11 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
     const bool scales = m.kind == MCQ_MODEL_GBM || m.kind == MCQ_MODEL_HESTON || m.kind == MCQ_MODEL_DUPIRE;
     const double dS = scales ? m.S0 / (double)k.S0 - 1.0 : 0.0, dK = (p.K - (double)k.K) - p.K * dS;
     k.dK = std::isfinite(dK) && std::fabs(dK) < 1e-6 * std::fabs(p.K) ? (float)dK : 0.f;
+    // prices below 2^104, subnormal ones among them, where the path starts below 2^-60; from 2^-125 up otherwise
+    const bool tiny = k.S0 < 0x1p-60f;
+    k.geo_win = tiny ? 150u << 23 : 126u << 23;
+    k.geo_low = tiny ? 1u : 2u << 23;
+    k.geo_span = (tiny ? 231u << 23 : 255u << 23) - k.geo_low;
     k.B = (float)p.B;
     k.pay_T = (float)p.T;
     switch (p.kind) {

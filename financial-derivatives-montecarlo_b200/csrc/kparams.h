@@ -93,6 +93,8 @@ struct KParams {
     float dK;                                      // K - (float)K, less K (S0 / (float)S0 - 1) where paths scale with S0
     float dcorr_f, dcorr_c;                        // what rounding the two corrections left out
     float pay_T;                                   // payoff maturity (discount sensitivity)
+    // geometric average: exponent bits of the running product's mantissa, smallest price and range as float bits
+    uint32_t geo_win, geo_low, geo_span;
     // ---- control variate / importance sampling
     float beta_cv, E_ctrl, z_star;
     float ctrl_sigma;                              // GBM control volatility (EST_CV_DUPIRE)

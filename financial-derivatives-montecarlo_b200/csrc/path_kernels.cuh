@@ -381,40 +381,41 @@ struct Leg {
     float S, V, r0, r1, tp;
     // Geometric average: the running product, its mantissa in r0 (1 <= r0 < 2) and its exponent in ge, one
     // logarithm per path instead of one per step (42.8 -> 21.1 instructions per path-step of the GBM
-    // pass).  The product's n roundings of 2^-24 stay below those of n logarithms and their sum.  gu: the
-    // largest bits(S) - bits(2^-126); beyond kGeomBits some S was not a normal positive float below 2^126
-    // (payoff()).
+    // pass).  The product's n roundings of 2^-24 stay below those of n logarithms and their sum.  The mantissa is
+    // kept in [2^a, 2^(a+1)), a from S0 (KParams::geo_win): from [1/2, 1) every price from 2^-125 to the largest float
+    // has a normal product, from [2^23, 2^24) every positive one below 2^104.  gu: the largest bits(S) - geo_low; from
+    // geo_span on, some price was none of these.  (A branch that scales such prices one by one: 856 -> 1032 us for GBM
+    // and 1261 -> 2352 us for PCA, 32 x 2^17 paths of 256 steps.)
     int ge;
     uint32_t gu;
-    static constexpr uint32_t kGeomBits = 0x7e000000u;
     static constexpr bool SUM = (PAY == PAY_ASIAN);
     __device__ __forceinline__ void init(const KParams& p) {
         S = p.S0; V = p.v0; r1 = 0.f; tp = 0.f;
-        r0 = (PAY == PAY_LOOKBACK || PAY == PAY_DOWNOUT) ? p.S0 : PAY == PAY_GEOM ? 1.f : 0.f;
-        ge = 0;
+        r0 = (PAY == PAY_LOOKBACK || PAY == PAY_DOWNOUT) ? p.S0 : PAY == PAY_GEOM ? __uint_as_float(p.geo_win) : 0.f;
+        ge = 127 - (int)(p.geo_win >> 23);
         gu = 0;
     }
-    __device__ __forceinline__ void multiply(bool on) {
-        const uint32_t b = __float_as_uint(r0 * S), u = __float_as_uint(S) - 0x00800000u;
+    __device__ __forceinline__ void multiply(const KParams& p, bool on) {
+        const uint32_t b = __float_as_uint(r0 * S), u = __float_as_uint(S) - p.geo_low;
         if (on) {
-            ge += (int)(b >> 23) - 127;
-            r0 = __uint_as_float((b & 0x007fffffu) | 0x3f800000u);
+            ge += (int)(b >> 23) - (int)(p.geo_win >> 23);
+            r0 = __uint_as_float((b & 0x007fffffu) | p.geo_win);
             gu = max(gu, u);
         }
     }
     __device__ __forceinline__ void flush() {
         if constexpr (SUM) { kadd(r0, r1, tp); tp = 0.f; }
     }
-    __device__ __forceinline__ void update() {
+    __device__ __forceinline__ void update(const KParams& p) {
         if constexpr (PAY == PAY_ASIAN) tp += S;
-        else if constexpr (PAY == PAY_GEOM) multiply(true);
+        else if constexpr (PAY == PAY_GEOM) multiply(p, true);
         else if constexpr (PAY == PAY_LOOKBACK || PAY == PAY_DOWNOUT) r0 = fminf(r0, S);
         else if constexpr (PAY == PAY_UPOUT) r0 = fmaxf(r0, S);
     }
     // update() when `on`, as selects rather than a branch per step (the same values)
-    __device__ __forceinline__ void update_if(bool on) {
+    __device__ __forceinline__ void update_if(const KParams& p, bool on) {
         if constexpr (PAY == PAY_ASIAN) tp += on ? S : 0.f;
-        else if constexpr (PAY == PAY_GEOM) multiply(on);
+        else if constexpr (PAY == PAY_GEOM) multiply(p, on);
         else if constexpr (PAY == PAY_LOOKBACK || PAY == PAY_DOWNOUT) r0 = on ? fminf(r0, S) : r0;
         else if constexpr (PAY == PAY_UPOUT) r0 = on ? fmaxf(r0, S) : r0;
     }
@@ -456,23 +457,24 @@ struct Leg {
             inc = (p.mil != 0.f) ? fmaf(p.mil, fmaf(dw2, dw2, -hstep), inc) : inc;
             V = V + inc;
         }
-        if constexpr (RUN && path_dep<PAY>()) update();
+        if constexpr (RUN && path_dep<PAY>()) update(p);
     }
     // GBM step from a raw normal: S + S (mu h + (sigma sqrt h) z)
-    __device__ __forceinline__ void step_gbm_z(float z, float sig_sqh, float muh) {
-        S = fmaf(S, fmaf(sig_sqh, z, muh), S);
-        if constexpr (path_dep<PAY>()) update();
+    __device__ __forceinline__ void step_gbm_z(const KParams& p, float z, float muh) {
+        S = fmaf(S, fmaf(p.sig_sqh, z, muh), S);
+        if constexpr (path_dep<PAY>()) update(p);
     }
     // 2^((ge + log2 r0) / n) = 2^q 2^f, q the exponent's integer part and 2^f, 0 <= f <= 1, a polynomial in f - c
     // whose constant 2^c is a float to 1e-5 ulp (fit error 2.5e-9): every path's mean lies in the same narrow
     // range, so an inverse of n or an exponential a little off would bias them all alike.  A path that met a
-    // zero, negative or undefined price has no geometric mean (NaN, payoff 0, as the exp of a sum of
-    // logarithms gives for all but the zero, whose payoff is 0 as well); one that is infinite at its end has an
-    // infinite one.
-    __device__ __forceinline__ float geometric_mean(int n) const {
-        if (gu >= kGeomBits) return S == __int_as_float(0x7f800000) ? S : __int_as_float(0x7fffffff);
-        const int q = (int)floorf((float)ge / (float)n);
-        const float d = ((float)(ge - q * n) + log2f(r0)) / (float)n - 0x1.00061ap-1f;
+    // zero, negative, infinite or undefined price (or one outside the product's range) has no geometric mean (NaN,
+    // payoff 0), as the compensated sum of logarithms, one of them infinite or undefined, has none.
+    __device__ __forceinline__ float geometric_mean(const KParams& p, int n) const {
+        if (gu >= p.geo_span) return __int_as_float(0x7fffffff);
+        const int g = ge + (int)(p.geo_win >> 23) - 127;
+        const float r = __uint_as_float((__float_as_uint(r0) & 0x007fffffu) | 0x3f800000u);
+        const int q = min((int)floorf((float)g / (float)n), 127), qn = max(q, -126);
+        const float d = ((float)(g - q * n) + log2f(r)) / (float)n - 0x1.00061ap-1f;
         float e = 0x1.c939fcp-13f;
         e = fmaf(e, d, 0x1.f0e27cp-10f);
         e = fmaf(e, d, 0x1.bdbaf4p-7f);
@@ -480,7 +482,7 @@ struct Leg {
         e = fmaf(e, d, 0x1.5be578p-2f);
         e = fmaf(e, d, 0x1.f5e88cp-1f);
         e = fmaf(e, d, 0x1.6a0ce4p+0f);
-        return e * __int_as_float((q + 127) << 23);
+        return e * __int_as_float((qn + 127) << 23) * __int_as_float((q - qn + 127) << 23);
     }
     // X - K less what rounding S0 and K to single precision left in the difference (KParams::dK): it shifts
     // every path's payoff alike, so it costs an option at the money 10 to 30 times its relative size.
@@ -491,7 +493,7 @@ struct Leg {
     __device__ __forceinline__ float payoff(const KParams& p, int n, float corr, float dcorr) const {
         if constexpr (PAY == PAY_EUR || PAY == PAY_BASKET) return over_strike(p, S) * p.disc;
         else if constexpr (PAY == PAY_ASIAN) return over_strike(p, (r0 - r1) / (float)n);
-        else if constexpr (PAY == PAY_GEOM) return over_strike(p, geometric_mean(n));
+        else if constexpr (PAY == PAY_GEOM) return over_strike(p, geometric_mean(p, n));
         else if constexpr (PAY == PAY_LOOKBACK) return fmaf(-r0, dcorr, fmaf(-r0, corr, S));
         else if constexpr (PAY == PAY_UPOUT) return (r0 / corr >= p.B) ? 0.f : over_strike(p, S) * p.disc;
         else return (r0 * corr <= p.B) ? 0.f : over_strike(p, S) * p.disc;   // PAY_DOWNOUT
@@ -526,7 +528,7 @@ struct PathC {
         const float t = (float)k * p.dup_f;
         if constexpr (HES && COUPLED) {   // run_upd is a runtime flag only here
             f.template step<false>(p, dw1, dw2, t, muh_f, p.om_f, p.h, k);
-            if constexpr (path_dep<PAY>()) f.update_if(run_upd);
+            if constexpr (path_dep<PAY>()) f.update_if(p, run_upd);
         } else {
             f.template step<true>(p, dw1, dw2, t, muh_f, p.om_f, p.h, k);
         }
@@ -541,7 +543,7 @@ struct PathC {
         const float tc = (float)ck * p.dup_c;
         if constexpr (HES) {
             c.template step<false>(p, a1, a2, tc, muh_c, p.om_c, p.hc, ck);
-            if constexpr (path_dep<PAY>()) c.update_if(run_upd);
+            if constexpr (path_dep<PAY>()) c.update_if(p, run_upd);
         } else {
             c.template step<true>(p, a1, a2, tc, muh_c, p.om_c, p.hc, ck);
         }
@@ -611,7 +613,7 @@ struct PathC {
                 }
             } else if constexpr (MOD == MOD_GBM && !COUPLED) {
 #pragma unroll
-                for (int i = 0; i < 32; i++) f.step_gbm_z(z[i], p.sig_sqh, muh_f);
+                for (int i = 0; i < 32; i++) f.step_gbm_z(p, z[i], muh_f);
                 k += 32;
             } else if constexpr (COUPLED) {
                 if (m == 0 && p.M == 2) {

@@ -50,7 +50,9 @@ extern "C" {
 /* Payoff kinds.  0..5 follow PayoffKind (methods_cuda.cu:202); 6 is an engine addition. */
 #define MCQ_PAYOFF_EUROPEAN          0  /* payoffs.hpp:14 */
 #define MCQ_PAYOFF_ASIAN             1  /* payoffs.hpp:15 (undiscounted, as the reference) */
-#define MCQ_PAYOFF_GEOM_ASIAN        2  /* payoffs.hpp:16 (undiscounted) */
+#define MCQ_PAYOFF_GEOM_ASIAN        2  /* payoffs.hpp:16 (undiscounted).  A path with a price that is not
+                                           positive and finite pays 0, as does one with a positive price
+                                           below 2^-125 (S0 below 2^-60: a price from 2^104 up) */
 #define MCQ_PAYOFF_LOOKBACK          3  /* payoffs.hpp:17 floating strike, undiscounted */
 #define MCQ_PAYOFF_BARRIER_UP_OUT    4  /* payoffs.hpp:18 */
 #define MCQ_PAYOFF_BASKET            5  /* payoffs.hpp:19 */
