@@ -130,9 +130,13 @@ void shutdown_engine() {
     E.ready = false;
 }
 
+// What the engine keeps between calls for speed alone (the book's normals, the adjoint's paths) counts as
+// free: drivers size their first pass by this figure, and a call's result is not to depend on what ran before.
 long long gpu_free_bytes_80() {   // gpu_free_bytes, methods_cuda.cu:258-263
     size_t f = 0, t = 0;
     MCQ_CUDA(cudaMemGetInfo(&f, &t));
+    for (auto& b : engine().store_slabs) f += b->cap;
+    for (auto& w : engine().pool) f += w->paths.cap;
     return (long long)((double)f * 0.8);
 }
 
@@ -757,7 +761,8 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
     const size_t per_block = (size_t)warps * adjoint_path_bytes(k.model, n_steps);
     for (;;) {
         try {
-            k.path_scratch = (float4*)ws.paths.ensure((size_t)blocks * per_block);
+            // whole pages, so that cap is what the device has given (gpu_free_bytes_80)
+            k.path_scratch = (float4*)ws.paths.ensure(((size_t)blocks * per_block + kDevicePage - 1) / kDevicePage * kDevicePage);
             break;
         } catch (const Error&) {
             if (blocks == 1) throw;

@@ -34,6 +34,8 @@ struct Error : std::runtime_error {
 #define MCQ_REQUIRE(cond, code, msg) \
     do { if (!(cond)) throw ::mcq::Error((code), (msg)); } while (0)
 
+constexpr size_t kDevicePage = (size_t)2 << 20;   // the granularity of large device allocations
+
 // Grow-only device / pinned-host buffers.
 struct DevBuf {
     void* p = nullptr;
