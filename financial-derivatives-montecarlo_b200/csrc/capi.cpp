@@ -394,18 +394,29 @@ int mcq_qmc_pass_device(const mcq_model* m, const mcq_payoff* p, int n_steps, in
     NEED(sums_device);
     PassArgs a = qmc_args(m, p, n_steps, noise_mode, bb, pca, salt_base, R, offset, n_points, flags);
     ensure_ready();
+    const unsigned long long last = engine().device_stream;
     Workspace& ws = engine().ws(0);
     cudaStream_t user = (cudaStream_t)stream;
     if (user) {
-        // run on the caller's stream: swap it in for this call
+        // run on the caller's stream: swap it in for this call.  The workspace's scratch, direction words
+        // and status word are used on the caller's stream: it waits for what earlier calls left on the
+        // workspace, and later work on the workspace (the next pass, the status read of the next
+        // synchronous call) waits for this pass
+        unsigned long long id = 0;
+        MCQ_CUDA(cudaStreamGetId(user, &id));
+        if (id + 1 != last) lend_to_caller_stream(ws, user);
         cudaStream_t own = ws.stream;
         ws.stream = user;
-        try { pass_async(ws, a, sums_device); } catch (...) { ws.stream = own; throw; }
+        try {
+            pass_async(ws, a, sums_device);
+        } catch (...) {
+            ws.stream = own;
+            join_caller_stream(ws, user);
+            throw;
+        }
         ws.stream = own;
-        // the workspace's scratch and status word were used on the caller's stream: later work
-        // on the workspace (the next pass, the status read of the next synchronous call) waits
-        // for this pass
         join_caller_stream(ws, user);
+        engine().device_stream = id + 1;
     } else {
         pass_async(ws, a, sums_device);
     }

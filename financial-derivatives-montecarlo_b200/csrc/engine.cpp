@@ -69,6 +69,15 @@ Workspace::~Workspace() {
     if (stream) cudaStreamDestroy(stream);
 }
 
+void lend_to_caller_stream(Workspace& ws, cudaStream_t caller) {
+    cudaStreamCaptureStatus cs;
+    MCQ_CUDA(cudaStreamIsCapturing(caller, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return;   // (a wait across the capture's boundary is an error)
+    if (!ws.joined) MCQ_CUDA(cudaEventCreateWithFlags(&ws.joined, cudaEventDisableTiming));
+    MCQ_CUDA(cudaEventRecord(ws.joined, ws.stream));
+    MCQ_CUDA(cudaStreamWaitEvent(caller, ws.joined, 0));
+}
+
 void join_caller_stream(Workspace& ws, cudaStream_t caller) {
     if (!ws.joined) MCQ_CUDA(cudaEventCreateWithFlags(&ws.joined, cudaEventDisableTiming));
     MCQ_CUDA(cudaEventRecord(ws.joined, caller));
@@ -85,6 +94,7 @@ Engine& engine() {
 Workspace& Engine::ws(int i) {
     while ((int)pool.size() <= i) pool.emplace_back(new Workspace());
     pool[i]->ensure_stream();
+    device_stream = 0;
     return *pool[i];
 }
 

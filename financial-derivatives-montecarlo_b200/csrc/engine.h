@@ -54,9 +54,9 @@ struct PinnedBuf {
 
 // Scratch owned by one stream: item partials, per-replica sums, scrambled direction words,
 // small parameter uploads.  Launches on one workspace are ordered by its stream; a pass run on a
-// caller's stream is joined back into it (`joined`, recorded on the caller's stream and waited
-// on by the workspace stream), so later work on the workspace, and the read of its status word,
-// comes after that pass.
+// caller's stream first waits for it and is joined back into it (event `joined`), so such a pass comes after
+// earlier work on the workspace, whatever stream that ran on, and later work, and the read of the
+// status word, after the pass.
 struct Workspace {
     cudaStream_t stream = nullptr;
     cudaEvent_t joined = nullptr;
@@ -129,6 +129,8 @@ struct Engine {
     std::unordered_map<uint64_t, TuneState> tune;
     std::vector<std::unique_ptr<DevBuf>> store_slabs;   // the book's stored normals (book.cu)
     bool store_busy = false;                            // a batched book is running on them
+    unsigned long long device_stream = 0;            // 1 + id of the caller's stream that workspace 0's last work ran on
+                                                     // (0: another; cleared by every use of a workspace)
     int launches = 0;                                // kernel launches issued (accounting)
     int last_gpi = 0, last_carry = 0;                // work layout of the last fused pass
     Workspace& ws(int i);
@@ -195,6 +197,8 @@ std::vector<double> pass_sync(Workspace& ws, const PassArgs& a);
 // After a synchronisation of ws.stream: raises MCQ_ERR_TIMEOUT if a bounded device-side wait of
 // the workspace's last tensor-core or assisted pass gave up.
 void check_err_word(Workspace& ws);
+// Orders `caller` after what earlier calls left on the workspace: its own work and, through it, other callers'.
+void lend_to_caller_stream(Workspace& ws, cudaStream_t caller);
 // Orders the workspace stream after everything issued so far on `caller`.
 void join_caller_stream(Workspace& ws, cudaStream_t caller);
 // The workspace's error word for a pass with bounded device waits (cleared unless it still holds
