@@ -760,9 +760,10 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
         MCQ_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(double) * n_nodes, ws.stream));
     }
     k.node_out = d_nodes;
-    const size_t smem = adjoint_smem_bytes(k.model, n_steps, n_nodes);
-    k.node_copies_log2 = adjoint_node_copies_log2(k.model, n_steps, n_nodes);
-    const int warps = adjoint_warps(k.model);
+    const AdjointShape shape = adjoint_shape(k.model, n_steps, n_nodes);
+    k.node_copies_log2 = shape.node_copies_log2;
+    const int warps = shape.warps;
+    const size_t smem = shape.smem;
     KernelInfo& ki = kernel_info(fn, smem, warps * 32);
     // items are dealt to the CTAs in turn, one warp of each first
     long long blocks = std::min<long long>((long long)k.n_items, (long long)ki.blocks_per_sm * E.sm_count);

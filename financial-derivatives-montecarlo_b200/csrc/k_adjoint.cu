@@ -88,6 +88,8 @@ __device__ __forceinline__ float local_sigma(const KParams& p, float S, int k, c
 // One CTA of 24 warps per SM (80 registers) rather than three of eight, so that the node array can hold
 // several copies: a float atomic on shared memory is a compare-and-swap loop that goes round once for
 // each lane of the warp on the same node, and the paths of a warp share cells (all of them in the first steps).
+// Where one copy does not fit beside 24 warps' tiles and start words (1024 steps and more than 3836 nodes: 233 KB at
+// 4096) a launch takes 16 (213 KB with four copies).
 constexpr int kAdjWarps = 24;
 constexpr int kAdjThreads = kAdjWarps * 32;
 constexpr size_t kAdjSmemMax = 227 * 1024;
@@ -117,11 +119,11 @@ template <int MOD, int PAY>
 __global__ void __launch_bounds__(kAdjThreads, 1) k_adjoint(const __grid_constant__ KParams p) {
     extern __shared__ float4 smem4[];
     grid_dependency_wait();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int N = p.n_steps;
     float* buf = reinterpret_cast<float*>(smem4) + wib * 1024;       // 32 x 32 transpose tile
     // FP32 node sums of the CTA, 2^lc copies of each node side by side, lane l adding to copy l mod 2^lc
-    float* nodes = reinterpret_cast<float*>(smem4) + kAdjWarps * 1024;
+    float* nodes = reinterpret_cast<float*>(smem4) + warps * 1024;
     const int lc = p.node_copies_log2;
     const int node_floats = (MOD == MOD_LVGRID) ? (((p.lv_nK * p.lv_nt << lc) + 3) & ~3) : 0;
     float* my_nodes = nodes + (lane & ((1 << lc) - 1));
@@ -130,17 +132,17 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adjoint(const __grid_constan
     // each tile's Sobol start word, carried from group to group: slot 32 t + lane
     uint32_t* carry = reinterpret_cast<uint32_t*>(nodes + node_floats + trow_floats) + wib * N;
     Pending* pend = reinterpret_cast<Pending*>(reinterpret_cast<uint32_t*>(nodes + node_floats + trow_floats) +
-                                               kAdjWarps * N) + wib * 64;
+                                               warps * N) + wib * 64;
     if constexpr (MOD == MOD_LVGRID) {
         for (int i = threadIdx.x; i < node_floats; i += blockDim.x) nodes[i] = 0.f;
         for (int k = threadIdx.x; k <= N; k += blockDim.x) trow[k] = lv_time_row(p, k);
         __syncthreads();
     }
     const float h = p.h, sqh = p.sqrt_h, muh = p.mu * p.h;
-    const int total_warps = gridDim.x * kAdjWarps;   // a small call's items go to different SMs first
+    const int total_warps = gridDim.x * warps;   // a small call's items go to different SMs first
     // two path stretches, used in turn: steps 2q and 2q + 1 of lane l as {S, z, S, z} at [32 q + l]
     const size_t stretch = (size_t)(N / 2 * 32);
-    float4* paths = p.path_scratch + (size_t)(blockIdx.x * kAdjWarps + wib) * (2 * stretch);
+    float4* paths = p.path_scratch + (size_t)(blockIdx.x * warps + wib) * (2 * stretch);
     const uint64_t gend_all = p.g0 + p.G;
     for (int item = wib * gridDim.x + blockIdx.x; item < p.n_items; item += total_warps) {
         const int r = item / p.items_per_rep;
@@ -458,25 +460,25 @@ const void* lookup_adjoint(int model, int payoff) {
     }
 }
 
-int adjoint_warps(int model) { return model == MOD_HESTON ? kWarpsPerBlock : kAdjWarps; }
-
-static size_t adjoint_smem(int model, int n_steps, int n_nodes, int lc) {
+// Shared memory of `warps` warps with 2^lc copies of the nodes: tiles, start words, lists, nodes, time rows.
+static size_t adjoint_smem(int model, int warps, int n_steps, int n_nodes, int lc) {
     const int D = (model == MOD_HESTON ? 2 : 1) * n_steps;
     const size_t trow = (model == MOD_LVGRID) ? (size_t)((2 * (n_steps + 1) + 3) & ~3) : 0;
     const size_t nodes = (size_t)(((n_nodes << lc) + 3) & ~3);
     const size_t pend = model == MOD_HESTON ? 0 : 64 * sizeof(Pending) / sizeof(float);
-    return (adjoint_warps(model) * (1024 + (size_t)D + pend) + nodes + trow) * sizeof(float);   // tile, start words, list
+    return (warps * (1024 + (size_t)D + pend) + nodes + trow) * sizeof(float);
 }
 
-// eight copies of each node where they fit beside the warps' tiles and start words
-int adjoint_node_copies_log2(int model, int n_steps, int n_nodes) {
-    int lc = 3;
-    while (lc > 0 && adjoint_smem(model, n_steps, n_nodes, lc) > kAdjSmemMax) lc--;
-    return lc;
-}
-
-size_t adjoint_smem_bytes(int model, int n_steps, int n_nodes) {
-    return adjoint_smem(model, n_steps, n_nodes, adjoint_node_copies_log2(model, n_steps, n_nodes));
+AdjointShape adjoint_shape(int model, int n_steps, int n_nodes) {
+    AdjointShape a;
+    a.warps = model == MOD_HESTON ? kWarpsPerBlock : kAdjWarps;
+    while (a.warps > 8 && adjoint_smem(model, a.warps, n_steps, n_nodes, 0) > kAdjSmemMax) a.warps -= 8;
+    // eight copies of each node where they fit beside the warps' tiles and start words
+    a.node_copies_log2 = 3;
+    while (a.node_copies_log2 > 0 && adjoint_smem(model, a.warps, n_steps, n_nodes, a.node_copies_log2) > kAdjSmemMax)
+        a.node_copies_log2--;
+    a.smem = adjoint_smem(model, a.warps, n_steps, n_nodes, a.node_copies_log2);
+    return a;
 }
 
 size_t adjoint_path_bytes(int model, int n_steps) {
