@@ -805,6 +805,7 @@ struct BookRunner {
         }
         float* p = (float*)((char*)slabs[slab]->p + slab_at);
         slab_at += bytes;
+        engine().store_used = slab + 1;
         return p;
     }
 
@@ -832,8 +833,9 @@ struct BookRunner {
                 }
             if (drawn < 4.0 * (double)(upto - stored_pts[l]) * (double)dims) continue;
             if (!d_stored) {
-                d_stored = &engine().ws(1).xbuf[5];
-                grow(*d_stored, sizeof(float*) * (size_t)(kBookMaxLevels * kStoreMaxBlocks));
+                DevBuf& t = engine().ws(1).xbuf[5];
+                try { grow(t, sizeof(float*) * (size_t)(kBookMaxLevels * kStoreMaxBlocks)); } catch (const Error&) { return; }
+                d_stored = &t;
                 h_stored.assign((size_t)kBookMaxLevels * kStoreMaxBlocks, nullptr);
             }
             const size_t bytes = sizeof(float) * (size_t)R * (size_t)dims * kStorePoints;
@@ -1112,9 +1114,8 @@ struct BookRunner {
         Slot s(E.ws(0));
         struct Busy {
             Engine& e;
-            ~Busy() { e.store_busy = false; }
+            ~Busy() { e.store_used = 0; }
         } busy{E};
-        E.store_busy = true;
         constexpr int kSide = kBookClasses - 1;   // class 0 runs on the main stream
         cudaStream_t side[kSide];
         cudaEvent_t fork = nullptr, join[kSide] = {};

@@ -683,6 +683,14 @@ int mcq_debug_wait_timeout(uint32_t polls) {
     API_END
 }
 
+int mcq_debug_device_memory(int64_t limit, int64_t* held) {
+    API_BEGIN
+    MCQ_REQUIRE(limit >= 0, MCQ_ERR_INVALID, "negative limit");
+    engine().device_limit = (size_t)limit;
+    if (held) *held = (int64_t)engine().device_held;
+    API_END
+}
+
 int mcq_debug_last_pass_layout(int* groups_per_item, int* carry_words) {
     API_BEGIN
     MCQ_REQUIRE(groups_per_item && carry_words, MCQ_ERR_INVALID, "NULL argument");

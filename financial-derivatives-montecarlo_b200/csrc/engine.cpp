@@ -23,12 +23,16 @@ void* DevBuf::ensure(size_t bytes) {
     if (bytes <= cap && p) return p;
     release();
     size_t want = std::max<size_t>(bytes, 256);
-    cudaError_t e = cudaMalloc(&p, want);
     Engine& E = engine();
-    if (e == cudaErrorMemoryAllocation && !E.store_busy && !E.store_slabs.empty()) {
-        cudaGetLastError();   // an earlier book's normals give way to the call that needs the memory
-        E.store_slabs.clear();
-        e = cudaMalloc(&p, want);
+    auto alloc = [&] {
+        if (E.device_limit && E.device_held + want > E.device_limit) return cudaErrorMemoryAllocation;
+        return cudaMalloc(&p, want);
+    };
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation) {
+        p = nullptr;
+        cudaGetLastError();
+        if (E.give_back_idle()) e = alloc();
     }
     if (e != cudaSuccess) {
         p = nullptr;
@@ -36,10 +40,14 @@ void* DevBuf::ensure(size_t bytes) {
         throw Error(MCQ_ERR_NOMEM, "device allocation of " + std::to_string(want) + " bytes failed");
     }
     cap = want;
+    E.device_held += cap;
     return p;
 }
 void DevBuf::release() {
-    if (p) cudaFree(p);
+    if (p) {
+        cudaFree(p);
+        engine().device_held -= cap;
+    }
     p = nullptr;
     cap = 0;
 }
@@ -89,6 +97,16 @@ void join_caller_stream(Workspace& ws, cudaStream_t caller) {
 Engine& engine() {
     static Engine e;
     return e;
+}
+
+// Memory kept between calls for speed alone gives way to a call that needs it: the slabs that no running book has
+// blocks in, and the adjoint's path scratch (an adjoint takes it after its other device buffers, so none is running
+// on it when a buffer grows).
+bool Engine::give_back_idle() {
+    const size_t held = device_held;
+    if (store_slabs.size() > store_used) store_slabs.resize(store_used);
+    for (auto& w : pool) w->paths.release();
+    return device_held < held;
 }
 
 Workspace& Engine::ws(int i) {

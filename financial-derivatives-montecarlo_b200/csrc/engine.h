@@ -128,7 +128,9 @@ struct Engine {
     std::unordered_set<const void*> kattr;           // kernels whose smem limit is raised
     std::unordered_map<uint64_t, TuneState> tune;
     std::vector<std::unique_ptr<DevBuf>> store_slabs;   // the book's stored normals (book.cu)
-    bool store_busy = false;                            // a batched book is running on them
+    size_t store_used = 0;                              // how many of them the running book has blocks in
+    bool give_back_idle();
+    size_t device_held = 0, device_limit = 0;           // bytes of all DevBufs; most they may hold (0: what the device has)
     unsigned long long device_stream = 0;            // 1 + id of the caller's stream that workspace 0's last work ran on
                                                      // (0: another; cleared by every use of a workspace)
     int launches = 0;                                // kernel launches issued (accounting)

@@ -275,8 +275,9 @@ int mcq_run_is(const mcq_model* gbm, const mcq_payoff* european, double z_star, 
  * step with MCQ_FLAG_HESTON_MILSTEIN); node_vega (optional, lv_nt * lv_nK doubles, same layout
  * as lv_sigma) receives dV/dsigma(K_i, t_j).  Lipschitz payoffs only: European, arithmetic Asian,
  * lookback.  n_steps: multiple of 32 in [32, 1024] (Heston: of 16 in [16, 1024]); path states
- * go through a scratch array in device memory (up to 256 bytes a step for each resident warp, 512 for
- * Heston; kept until mcq_shutdown). */
+ * go through a scratch array in device memory (512 bytes a step for each resident warp: 0.93 GB at 512
+ * steps; kept until mcq_shutdown or until a call runs out of memory; where it is not to be had, fewer
+ * warps share the work). */
 int mcq_adjoint(const mcq_model* m, const mcq_payoff* p, int n_steps, uint32_t salt_base, int R,
                 uint32_t offset, int64_t n_points, int flags, mcq_greeks* out, double* node_vega);
 
@@ -288,7 +289,7 @@ int mcq_adjoint(const mcq_model* m, const mcq_payoff* p, int n_steps, uint32_t s
  * stream-per-level form (methods_cuda.cu:1745-1755) with the same kernels.  Both give
  * bit-identical results.  A batched book whose options share points keeps their normals in device
  * memory (as much as it fills, at most 16 GiB and an eighth of what is free; given back by
- * mcq_shutdown).  No counterpart in the reference (which rejects basket MLQMC,
+ * mcq_shutdown or to a call that runs out of memory).  No counterpart in the reference (which rejects basket MLQMC,
  * methods_cuda.cu:1695-1697).  stats may be NULL. */
 int mcq_book_price(const mcq_book_option* opts, int n, const mcq_mlmc_cfg* ml, const mcq_qmc_cfg* qc,
                    int mode, mcq_book_result* out, mcq_book_stats* stats);
@@ -396,6 +397,10 @@ int mcq_debug_pass_dump(const mcq_model* m, int n_steps, int noise_mode, mcq_han
    the Sobol start words each warp carries from group to group in shared memory (0: every tile
    walks its start word from the digital shift). */
 int mcq_debug_last_pass_layout(int* groups_per_item, int* carry_words);
+/* Device memory of the engine's buffers: *held (may be NULL) receives their bytes; from now on an allocation that
+   would take them above `limit` fails as on a full device (0: no limit).  For tests of calls that run short of
+   memory. */
+int mcq_debug_device_memory(int64_t limit, int64_t* held);
 /* The book kernel's per-replica sums over one slice of one option (level `level`, points
    offset .. offset + n_points - 1, R = qc->R replicas with salts qc->salt_base + level R + r):
    sums_host[R][20] = {sum dY, sum dY^2, sum Yf, sum Yf^2, sum d(dY)/dS0_a for a < 16 (0 beyond
