@@ -34,6 +34,7 @@
 #include <curand.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -63,7 +64,8 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
 unsigned char* g_scratch[kMaxDevices] = {};      // device address the table was loaded at
 unsigned long long g_ctx_id[kMaxDevices] = {};   // context it was loaded in (driver context id)
-int g_sm_count[kMaxDevices] = {};
+int g_sm_count[kMaxDevices] = {}, g_smem_optin[kMaxDevices] = {};
+std::atomic<int> g_last_gpi{0}, g_last_carry{0};   // work layout of the last call
 
 // The driver's id of the current context (unique for the life of the process: a context
 // created after a cudaDeviceReset has a new id), through the runtime's driver entry points.
@@ -93,7 +95,7 @@ unsigned long long current_context_id() {
 // Every call, with the device current: resolve the array's device address (the host-side name
 // g_noalloc_scratch is only a stand-in and must never be passed to a kernel), and load the
 // direction table when this device's array has not been loaded in this context at this address.
-unsigned char* scratch_for_current_device(int* sm_count) {
+unsigned char* scratch_for_current_device(int* sm_count, int* smem_optin) {
     int dev = -1;
     MCQ_CUDA(cudaGetDevice(&dev));
     MCQ_REQUIRE(dev >= 0 && dev < kMaxDevices, MCQ_ERR_RANGE, "device index beyond the set-up table");
@@ -108,13 +110,13 @@ unsigned char* scratch_for_current_device(int* sm_count) {
                         CURAND_STATUS_SUCCESS,
                     MCQ_ERR_INTERNAL, "curandGetDirectionVectors32 failed");
         MCQ_CUDA(cudaMemcpy(ptr, hv, kTableBytes, cudaMemcpyHostToDevice));
-        int sms = 0;
-        MCQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        g_sm_count[dev] = sms;
+        MCQ_CUDA(cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev));
+        MCQ_CUDA(cudaDeviceGetAttribute(&g_smem_optin[dev], cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         g_scratch[dev] = static_cast<unsigned char*>(ptr);
         g_ctx_id[dev] = ctx;
     }
     *sm_count = g_sm_count[dev];
+    *smem_optin = g_smem_optin[dev];
     return g_scratch[dev];
 }
 }  // namespace
@@ -169,8 +171,8 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
     k.R = R; k.gpi = (int)gpi; k.items_per_rep = (int)ipr; k.n_items = (int)(ipr * R);
     k.offset = a.offset; k.n_points = a.n_points; k.g0 = g0; k.G = G;
 
-    int sms = 0;
-    unsigned char* base = scratch_for_current_device(&sms);
+    int sms = 0, smem_optin = 0;
+    unsigned char* base = scratch_for_current_device(&sms, &smem_optin);
     const uint32_t* table = reinterpret_cast<const uint32_t*>(base);
     uint32_t* dirs = reinterpret_cast<uint32_t*>(base + kTableBytes);
     double* partials = reinterpret_cast<double*>(base + kTableBytes + kDirsBytes);
@@ -183,21 +185,24 @@ static void qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_step
     MCQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem));
     MCQ_REQUIRE(per_sm > 0, MCQ_ERR_INTERNAL, "kernel does not fit on an SM");
     // Sobol start words carried from group to group (one slot per 32-dimension tile), as the
-    // allocating pass does: when items hold several groups, the slots stay within the default
-    // 48 KB of dynamic shared memory (no attribute change) and keep the resident blocks per SM
+    // allocating pass does: when items hold several groups and the slots keep the resident blocks per SM.
+    // Beyond 48 KB (more than 12 tiles) the kernel's limit is raised to the device's, where the allocating
+    // passes have it too; that allocates nothing
     k.carry = 0;
     if (!packed && gpi >= 2) {
         const int words = 32 * ((D + 31) / 32);
         const size_t with = smem + (size_t)kWarpsPerBlock * words * sizeof(uint32_t);
         int per_sm_c = 0;
-        if (with <= 48 * 1024) {
-            MCQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, fn, kThreads, with));
-            if (per_sm_c >= per_sm) {
-                k.carry = words;
-                smem = with;
-            }
+        if (with > 48 * 1024)
+            MCQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin));
+        MCQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, fn, kThreads, with));
+        if (per_sm_c >= per_sm) {
+            k.carry = words;
+            smem = with;
         }
     }
+    g_last_gpi = k.gpi;
+    g_last_carry = k.carry;
     long long blocks = ((long long)k.n_items + kWarpsPerBlock - 1) / kWarpsPerBlock;
     blocks = std::min<long long>(blocks, (long long)per_sm * sms);
     blocks = std::max<long long>(blocks, 1);
@@ -225,4 +230,14 @@ extern "C" int mcq_qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int
         mcq::set_last_error(e.what());
         return MCQ_ERR_INTERNAL;
     }
+}
+
+extern "C" int mcq_debug_noalloc_layout(int* groups_per_item, int* carry_words) {
+    if (!groups_per_item || !carry_words) {
+        mcq::set_last_error("NULL argument");
+        return MCQ_ERR_INVALID;
+    }
+    *groups_per_item = mcq::g_last_gpi;
+    *carry_words = mcq::g_last_carry;
+    return MCQ_OK;
 }

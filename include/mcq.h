@@ -397,6 +397,8 @@ int mcq_debug_pass_dump(const mcq_model* m, int n_steps, int noise_mode, mcq_han
    the Sobol start words each warp carries from group to group in shared memory (0: every tile
    walks its start word from the digital shift). */
 int mcq_debug_last_pass_layout(int* groups_per_item, int* carry_words);
+/* The same of the last mcq_qmc_pass_noalloc of the process. */
+int mcq_debug_noalloc_layout(int* groups_per_item, int* carry_words);
 /* Device memory of the engine's buffers: *held (may be NULL) receives their bytes; from now on an allocation that
    would take them above `limit` fails as on a full device (0: no limit).  For tests of calls that run short of
    memory. */
