@@ -29,7 +29,7 @@ EXPORTS = [
     "mcq_run_mc_cv", "mcq_run_qmc_cv", "mcq_run_is", "mcq_qmc_pass", "mcq_qmc_pass_device",
     "mcq_mc_pass", "mcq_level_pass", "mcq_is_pass", "mcq_sobol_hh_u32", "mcq_sobol_hh_normal", "mcq_philox4x32_10",
     "mcq_bb_tables", "mcq_pca_matrix", "mcq_debug_pass_dump", "mcq_debug_wait_timeout",
-    "mcq_debug_last_pass_layout", "mcq_debug_device_memory", "mcq_debug_noalloc_layout", "mcq_qmc_pass_noalloc", "mcq_adjoint",
+    "mcq_debug_last_pass_layout", "mcq_debug_device_memory", "mcq_debug_book_stored", "mcq_debug_noalloc_layout", "mcq_qmc_pass_noalloc", "mcq_adjoint",
     "mcq_book_price", "mcq_book_level_sums", "mcq_book_create", "mcq_book_submit", "mcq_book_size",
     "mcq_book_run", "mcq_book_clear", "mcq_book_free",
 ]
@@ -375,6 +375,13 @@ def debug_device_memory(limit=0):
     held = C.c_int64()
     _check(lib().mcq_debug_device_memory(C.c_int64(limit), C.byref(held)))
     return held.value
+
+
+def debug_book_stored(level):
+    """Points of a level whose normals the last batched book stored."""
+    n = C.c_int64()
+    _check(lib().mcq_debug_book_stored(C.c_int(level), C.byref(n)))
+    return n.value
 
 
 def debug_noalloc_layout():

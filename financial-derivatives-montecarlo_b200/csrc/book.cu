@@ -1113,9 +1113,12 @@ struct BookRunner {
         Engine& E = engine();
         Slot s(E.ws(0));
         struct Busy {
-            Engine& e;
-            ~Busy() { e.store_used = 0; }
-        } busy{E};
+            BookRunner& b;
+            ~Busy() {
+                engine().store_used = 0;
+                engine().book_stored.assign(b.stored_pts, b.stored_pts + kBookMaxLevels);
+            }
+        } busy{*this};
         constexpr int kSide = kBookClasses - 1;   // class 0 runs on the main stream
         cudaStream_t side[kSide];
         cudaEvent_t fork = nullptr, join[kSide] = {};

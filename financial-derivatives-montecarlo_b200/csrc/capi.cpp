@@ -691,6 +691,14 @@ int mcq_debug_device_memory(int64_t limit, int64_t* held) {
     API_END
 }
 
+int mcq_debug_book_stored(int level, int64_t* points) {
+    API_BEGIN
+    NEED(points);
+    const auto& s = engine().book_stored;
+    *points = level >= 0 && level < (int)s.size() ? s[level] : 0;
+    API_END
+}
+
 int mcq_debug_last_pass_layout(int* groups_per_item, int* carry_words) {
     API_BEGIN
     MCQ_REQUIRE(groups_per_item && carry_words, MCQ_ERR_INVALID, "NULL argument");

@@ -129,6 +129,7 @@ struct Engine {
     std::unordered_map<uint64_t, TuneState> tune;
     std::vector<std::unique_ptr<DevBuf>> store_slabs;   // the book's stored normals (book.cu)
     size_t store_used = 0;                              // how many of them the running book has blocks in
+    std::vector<long long> book_stored;                 // points of each level that the last batched book stored
     bool give_back_idle();
     size_t device_held = 0, device_limit = 0;           // bytes of all DevBufs; most they may hold (0: what the device has)
     unsigned long long device_stream = 0;            // 1 + id of the caller's stream that workspace 0's last work ran on

@@ -399,6 +399,8 @@ int mcq_debug_pass_dump(const mcq_model* m, int n_steps, int noise_mode, mcq_han
 int mcq_debug_last_pass_layout(int* groups_per_item, int* carry_words);
 /* The same of the last mcq_qmc_pass_noalloc of the process. */
 int mcq_debug_noalloc_layout(int* groups_per_item, int* carry_words);
+/* Points of a level (from 0, per replica) whose normals the last MCQ_BOOK_BATCHED book stored. */
+int mcq_debug_book_stored(int level, int64_t* points);
 /* Device memory of the engine's buffers: *held (may be NULL) receives their bytes; from now on an allocation that
    would take them above `limit` fails as on a full device (0: no limit).  For tests of calls that run short of
    memory. */
