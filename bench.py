@@ -452,6 +452,42 @@ def adjoint_case(n_points, repeats=3):
                                        "delta": g["delta"], "rho": g["rho"], "vega": g["vega"]}}))
 
 
+def headline(full):
+    """The printed line: the metric with its checks, and one or two figures of each further workload.  It stays below
+    2,500 characters, so that whoever keeps only the end of the output still has it whole; the full record, with
+    every option's oracle comparison, goes to stderr."""
+    sd = lambda d: d["vs_oracle"]["error_in_se"] if d.get("vs_oracle") else None
+
+    def rnd(x):
+        if isinstance(x, dict):
+            return {k: rnd(v) for k, v in x.items()}
+        return [rnd(v) for v in x] if isinstance(x, list) else float("%.6g" % x) if isinstance(x, float) else x
+
+    line = {k: full[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+                                 "scaling", "vs_baseline", "dtype", "data", "config")}
+    more = {
+        "price_check": full["price_check"], "price_check_se": full["price_check_se"], "error_in_se": sd(full),
+        "geom_error_in_se": (full["geom_check"].get("vs_closed_form") or {}).get("error_in_se"),
+        "orderings": {k: {"value": v["value"], "ms_per_step": v["ms_per_step"], "error_in_se": sd(v)}
+                      for k, v in full["orderings"].items()},
+        "roofline": {k: full["roofline"][k] for k in ("bound", "achieved", "peak", "unit", "frac", "traffic")},
+    }
+    if "book" in full:
+        more["book_options_per_s"] = {k: [v[mode]["options_per_s"] for mode in ("batched", "plain") if mode in v]
+                                      for k, v in full["book"].items() if isinstance(v, dict) and "batched" in v}
+    if "other_workloads" in full:
+        more["other_workloads"] = {k: {"time_s": v["time_s"], "error_in_se": sd(v)}
+                                   for k, v in full["other_workloads"].items()}
+    line.update(rnd(more))
+    line["e2e"] = {k: full["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_run",
+                                               "n_samples", "converged")}
+    line["e2e"]["error_in_se"] = rnd(sd(full["e2e"]))
+    for k in ("gpu_launches", "clocks", "cpu_baseline"):
+        if k in full:
+            line[k] = full[k]
+    return line
+
+
 def run_reference(args):
     rank, _, world = dist_env()
     if rank != 0:
@@ -731,7 +767,8 @@ def main():
         line["other_workloads"] = others
     if world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline()
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)   # everything measured
+    print(json.dumps(headline(line)), flush=True)
 
 
 if __name__ == "__main__":
