@@ -39,7 +39,7 @@ struct LvEval {
 // Bilinear sigma(S, t) on the uniform grid exactly as the pricing pass's lv_sigma_row, with dsigma/dS
 // and the weights.  The time axis comes from the same per-step rows {j nK (as float bits), b}
 // (lv_time_row, path_kernels.cuh), which the CTA forms once in shared memory; the sweeps read them
-// instead of clamping, truncating and converting t in each of the three evaluations per step.
+// instead of clamping, truncating and converting t in both evaluations of a step.
 __device__ __forceinline__ LvEval lv_eval_row(const KParams& p, float S, float2 row) {
     LvEval e;
     float x = (S - p.lv_K0) * p.lv_inv_dK;
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adjoint(const __grid_constan
                 float S = p.S0, ts = 0.f, tot = 0.f, comp = 0.f, mn = p.S0;
                 int kmin = 0;
                 for (int d0 = 0; d0 < N; d0 += 32) {
-                    sobol_tile_plain(dr, N, d0 + lane, true, hg, p.u_cap, buf, lane, carry + d0 + lane, hg != gb ? 1 : 0);
+                    sobol_tile_plain(dr, N, d0 + lane, true, hg, p.u_cap, buf, lane, carry + d0 + lane, hg != gb);
                     __syncwarp();
                     // this lane's row of the tile, four steps per float4 (the swizzled layout makes row
                     // reads conflict-free), rolled over the chunks: fully unrolled, the sweeps overflowed
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_adjoint_heston(const __grid_con
             int kmin = 0;
             for (int t = 0; t < n_tiles; t++) {
                 sobol_tile_plain(dr, D, t * 32 + lane, true, hg, p.u_cap, buf, lane, carry + t * 32 + lane,
-                                 hg != gb ? 1 : 0);
+                                 hg != gb);
                 __syncwarp();
                 const float4* row4 = reinterpret_cast<const float4*>(buf + lane * 32);
 #pragma unroll 2

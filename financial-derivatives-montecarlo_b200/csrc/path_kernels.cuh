@@ -218,15 +218,13 @@ __device__ __forceinline__ void sobol_tile_slot(const uint32_t* __restrict__ dr,
 // cache of these kernels (book 641 -> 602 options/s).
 __device__ __forceinline__ void sobol_tile_plain(const uint32_t* __restrict__ dr, int D, int dim, bool active,
                                                  uint64_t h, float u_cap, float* buf, int lane,
-                                                 uint32_t* slot = nullptr, int cont = 0) {
+                                                 uint32_t* slot = nullptr, bool cont = false) {
     if (!active) return;
     const uint32_t* col = dr + dim;
     const uint32_t L0 = __ldg(col), L1 = __ldg(col + D), L2 = __ldg(col + 2 * D),
                    L3 = __ldg(col + 3 * D), L4 = __ldg(col + 4 * D);
     uint32_t x;
-    if (slot != nullptr && cont == 2) {
-        x = *slot;
-    } else if (slot != nullptr && cont) {
+    if (slot != nullptr && cont) {
         x = *slot ^ L4 ^ __ldg(col + (4 + __ffsll((long long)h)) * D);
     } else {
         x = __ldg(col + 32 * D);
