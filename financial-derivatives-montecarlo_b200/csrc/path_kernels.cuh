@@ -190,9 +190,10 @@ __device__ __forceinline__ void sobol_tile(const uint32_t* __restrict__ dr, int 
         std::make_integer_sequence<int, 32>{});
 }
 
-// The same with the slot as a pointer, for baskets whose steps do not fill a tile: there the address form's
-// volatile accesses cost
-// more than they save (5 assets x 52 steps x 16 x 2^16 paths: 346 us a call, 307 with this one).
+// The same with the slot as a pointer, for the baskets compiled for three CTAs per SM (up to eight assets): there the
+// address form's volatile accesses cost more than they save.  Address over pointer, 16 x 2^17 paths of about 260
+// dimensions, GBM / Dupire: 1 asset 1.013 / 1.025, 2 1.012 / 1.027, 4 1.081 / 1.038, 5 1.136 / 1.085, 7 1.164 / 1.069, 8
+// 1.122 / 1.060; 9 to 16 assets 0.98 to 1.01.
 __device__ __forceinline__ void sobol_tile_slot(const uint32_t* __restrict__ dr, int D, int dim, uint64_t h, float u_cap,
                                                 float* buf, int lane, uint32_t* slot, bool cont) {
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(buf) ^ ((uint32_t)lane << 2);
@@ -854,6 +855,7 @@ struct BasketTileC {
     static constexpr int NST = 2;
     static constexpr bool SMEM_TILE = true;
     static constexpr int TILE_DIMS = 32 / N * N;
+    static constexpr bool SLOT_POINTER = N <= 8;   // sobol_tile_slot
     float S[N];
     float muh;
     int k;
@@ -1161,6 +1163,10 @@ template <class C, class = void>
 struct tile_dims_of { static constexpr int value = 32; };
 template <class C>
 struct tile_dims_of<C, std::void_t<decltype(C::TILE_DIMS)>> { static constexpr int value = C::TILE_DIMS; };
+template <class C, class = void>
+struct slot_pointer_of { static constexpr bool value = false; };
+template <class C>
+struct slot_pointer_of<C, std::void_t<decltype(C::SLOT_POINTER)>> { static constexpr bool value = C::SLOT_POINTER; };
 template <class C>
 struct parity_of { static constexpr bool value = false; };
 template <>
@@ -1191,7 +1197,7 @@ __device__ __forceinline__ void run_group(const KParams& p, C& cons, const uint3
                 if constexpr (PLAIN)
                     sobol_tile_plain(dr, p.dstride, d0 + lane, lane < nv, h, p.u_cap, buf, lane,
                                      carry ? carry + s0 + lane : nullptr, cont);
-                else if constexpr (TD != 32)
+                else if constexpr (slot_pointer_of<C>::value)
                     sobol_tile_slot(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, carry ? carry + s0 + lane : nullptr, cont);
                 else
                     sobol_tile<PARITY>(dr, p.dstride, d0 + lane, h, p.u_cap, buf, lane, slots ? slots + 4 * s0 : 0, again);
