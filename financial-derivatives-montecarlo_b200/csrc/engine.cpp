@@ -388,7 +388,8 @@ void fill_params(Workspace& ws, const PassArgs& a, KParams& k) {
 // ------------------------------------------------------------------ launcher
 
 
-// Resident blocks per SM of kernel `fn` at `smem` bytes of dynamic shared memory.  A kernel's dynamic shared-memory limit is raised to the device's opt-in maximum
+// Resident blocks per SM of kernel `fn` at `smem` bytes of dynamic shared memory.  A kernel's dynamic shared-memory
+// limit is raised to the device's opt-in maximum
 // once, so that occupancy can be asked for several sizes (with and without carry slots) and any
 // of them launched.
 KernelInfo& kernel_info(const void* fn, size_t smem, int threads) {
@@ -826,7 +827,7 @@ void adjoint_run(const mcq_model& m, const mcq_payoff& p, int n_steps, uint32_t 
     out.n_paths = (int64_t)R * (int64_t)n_points;
     out.n_nodes = n_nodes;
     out.launches = E.launches - l0;
-    out.path_steps = 3.0 * (double)out.n_paths * n_steps;   // forward, path read back, reverse
+    out.path_steps = 3.0 * (double)out.n_paths * n_steps;   // forward, path read back, reverse (nominal: see mcq_greeks)
     if (node_vega)
         for (int i = 0; i < n_nodes; i++) node_vega[i] = nv[i] / (double)out.n_paths;
     out.time_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

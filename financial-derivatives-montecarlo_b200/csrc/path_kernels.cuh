@@ -379,7 +379,7 @@ struct Leg {
     // steps that flush() folds into the Kahan pair (r0, r1); extrema live in r0
     float S, V, r0, r1, tp;
     // Geometric average: the running product, its mantissa in r0 (1 <= r0 < 2) and its exponent in ge, one
-    // logarithm per path instead of one per step (42.8 -> 21.1 instructions per path-step of the GBM
+    // logarithm per path instead of one per step (42.8 -> 20.8 instructions per path-step of the GBM
     // pass).  The product's n roundings of 2^-24 stay below those of n logarithms and their sum.  The mantissa is
     // kept in [2^a, 2^(a+1)), a from S0 (KParams::geo_win): from [1/2, 1) every price from 2^-125 to the largest float
     // has a normal product, from [2^23, 2^24) every positive one below 2^104.  gu: the largest bits(S) - geo_low; from

@@ -166,7 +166,8 @@ typedef struct mcq_greeks {
     int32_t n_nodes;                              /* grid nodes written to node_vega (0 otherwise) */
     int32_t launches;
     double  time_s;
-    double  path_steps;                           /* three sweeps: forward, path read back, reverse */
+    double  path_steps;                           /* three sweeps of every path (forward, path read back,
+                                                     reverse), though one out of the money is swept once */
 } mcq_greeks;
 
 /* One option of a batched book (mcq_book_price), priced by MLQMC to its own eps.  Either
@@ -369,8 +370,9 @@ int mcq_qmc_pass_noalloc(const mcq_model* m, const mcq_payoff* p, int n_steps, u
  * Hong–Hickernell scrambled Sobol stream (methods_cuda.cu:753-825): out[d * n + i] for
  * dimension dim0 + d and point index offset + i.  _u32 returns the scrambled integers,
  * _normal their N(0,1) values with the reference's bits (normcdfinvf).  The priced passes take
- * the same u through one polynomial per 1/32 of the unit interval (the two end strata through
- * normcdfinvf): the same normals to their last places, no further from the exact quantile. */
+ * the same u through one polynomial per 1/32 of the unit interval (in the two end strata one in
+ * sqrt(-log2 t), t the distance to the nearer end): the same normals to their last places, no further
+ * from the exact quantile. */
 int mcq_sobol_hh_u32(uint32_t salt, int dim0, int nd, uint32_t offset, int64_t n,
                      uint32_t* out_host);
 int mcq_sobol_hh_normal(uint32_t salt, int dim0, int nd, uint32_t offset, int64_t n,
